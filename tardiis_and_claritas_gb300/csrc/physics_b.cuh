@@ -4,6 +4,7 @@
 #pragma once
 #include "physics_a.cuh"
 #include "device_scene.cuh"
+#include "visible_slope.cuh"
 
 namespace clr {
 namespace {  // header-only device code: internal linkage in every translation unit
@@ -17,6 +18,9 @@ enum {
     OF_SIDE_STATE = 33, OF_NONFINITE_DIRECTION = 34, OF_FRESNEL = 35, OF_HEIGHT_CNEXT_RANGE = 36,
     OF_HEIGHT_INVERSE_CDF = 37, OF_HEIGHT_OUTPUT = 38, OF_MICRO_WATCHDOG = 40
 };
+static_assert((int)OF_VNDF_PROJECTED_AREA == (int)SF_PROJECTED_AREA && (int)OF_VNDF_CDF == (int)SF_CDF &&
+                  (int)OF_VNDF_INVERSE_CDF == (int)SF_INVERSE_CDF,
+              "the slope sampler's failure codes");
 /* production failure codes and subcodes (:1844-1895) */
 enum {
     OP_OK = 0, OP_MICRO_NUMERICAL = 1, OP_MICRO_WATCHDOG = 2, OP_MACRO_GEOMETRY = 3, OP_MACRO_BOUNCE_LIMIT = 4,
@@ -38,36 +42,6 @@ enum {
 __device__ __forceinline__ double o_pos_inf(void) { return HUGE_VAL; }
 __device__ __forceinline__ void o_setf(int* code, int v) { if (code) *code = v; }
 
-/* B(x) = 1 - x sqrt(pi) erfcx(x) (:1925-1939) */
-__device__ double o_tail_B(double x) {
-    if (!(x >= 0.0) || !isfinite(x)) return -1.0;
-    const double SQRT_PI = 1.77245385090551602729816748334114518;
-    if (x < 5.0) {
-        double e = exp(x * x) * erfc(x);
-        double b = 1.0 - x * SQRT_PI * e;
-        return (isfinite(b) && b > 0.0) ? b : -1.0;
-    }
-    double y = 1.0 / (x * x);
-    double b = 0.5 * y - 0.75 * y * y + 1.875 * y * y * y - 6.5625 * y * y * y * y + 29.53125 * y * y * y * y * y -
-               162.421875 * y * y * y * y * y * y + 1055.7421875 * y * y * y * y * y * y * y;
-    return (isfinite(b) && b > 0.0) ? b : -1.0;
-}
-/* alpha=1 visible-slope marginal CDF, ordinary branch (:1944-1957) */
-__device__ int o_visible_cdf(double slope, double slope_i, double* out) {
-    if (!out || !isfinite(slope) || !isfinite(slope_i)) return 0;
-    if (slope >= slope_i) { *out = 1.0; return 1; }
-    const double K = 0.28209479177387814347403972578038629;
-    double q = K * exp(-slope_i * slope_i) + 0.5 * slope_i * erfc(-slope_i);
-    if (!(q > 0.0) || !isfinite(q)) return 0;
-    double n = K * exp(-slope * slope) + 0.5 * slope_i * erfc(-slope);
-    double f = n / q;
-    if (!isfinite(f)) return 0;
-    if (f < 0.0 && f > -1.0e-13) f = 0.0;
-    if (f > 1.0 && f < 1.0 + 1.0e-13) f = 1.0;
-    if (f < 0.0 || f > 1.0) return 0;
-    *out = f;
-    return 1;
-}
 /* signed-cot visible-slope sampler (:1965-2038) */
 __device__ int o_sample11(double slope_i, double U1, double U2, double* slope_x, double* slope_y, int* fc) {
     o_setf(fc, OF_NONE);
@@ -85,50 +59,8 @@ __device__ int o_sample11(double slope_i, double U1, double U2, double* slope_x,
     }
     if (!isfinite(slope_i)) { o_setf(fc, OF_VNDF_PROJECTED_AREA); return 0; }
     double sx = 0.0;
-    if (slope_i < -1.0) {
-        double x = -slope_i, Bx = o_tail_B(x);
-        if (!(Bx > 0.0) || !isfinite(Bx)) { o_setf(fc, OF_VNDF_PROJECTED_AREA); return 0; }
-        double target = log(u1), lo = 0.0, hi = fmax(1.0 / x, 1.0e-12);
-        int bracketed = 0;
-        for (int it = 0; it < 64; ++it) {
-            double y = x + hi, By = o_tail_B(y);
-            if (!(By > 0.0) || !isfinite(By)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            double Cc = hi / y + (x / y) * By;
-            if (!(Cc > 0.0) || !isfinite(Cc)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            double lr = -(2.0 * x * hi + hi * hi) + log(Cc / Bx);
-            if (!isfinite(lr)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            if (lr <= target) { bracketed = 1; break; }
-            hi *= 2.0;
-            if (!isfinite(hi)) { o_setf(fc, OF_VNDF_INVERSE_CDF); return 0; }
-        }
-        if (!bracketed) { o_setf(fc, OF_VNDF_INVERSE_CDF); return 0; }
-        for (int it = 0; it < 52; ++it) {
-            double mid = 0.5 * (lo + hi), y = x + mid, By = o_tail_B(y);
-            if (!(By > 0.0) || !isfinite(By)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            double Cc = mid / y + (x / y) * By;
-            if (!(Cc > 0.0) || !isfinite(Cc)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            double lr = -(2.0 * x * mid + mid * mid) + log(Cc / Bx);
-            if (!isfinite(lr)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            if (lr > target) lo = mid; else hi = mid;
-        }
-        sx = -(x + 0.5 * (lo + hi));
-    } else {
-        double lo = fmin(-1.0, slope_i - 1.0), hi = slope_i, flo = 1.0;
-        int bracketed = 0;
-        for (int it = 0; it < 64; ++it) {
-            if (!o_visible_cdf(lo, slope_i, &flo)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            if (flo <= u1) { bracketed = 1; break; }
-            lo = (lo < 0.0) ? 2.0 * lo : lo - 1.0;
-            if (!isfinite(lo)) { o_setf(fc, OF_VNDF_INVERSE_CDF); return 0; }
-        }
-        if (!bracketed) { o_setf(fc, OF_VNDF_INVERSE_CDF); return 0; }
-        for (int it = 0; it < 48; ++it) {
-            double mid = 0.5 * (lo + hi), fm = 0.0;
-            if (!o_visible_cdf(mid, slope_i, &fm)) { o_setf(fc, OF_VNDF_CDF); return 0; }
-            if (fm < u1) lo = mid; else hi = mid;
-        }
-        sx = 0.5 * (lo + hi);
-    }
+    int f2 = OF_NONE;
+    if (!o_visible_slope_x(slope_i, u1, &sx, &f2)) { o_setf(fc, f2); return 0; }
     double ey = 2.0 * u2 - 1.0;
     if (!(ey > -1.0 && ey < 1.0) || !isfinite(ey)) { o_setf(fc, OF_VNDF_INVERSE_CDF); return 0; }
     double sy = erfinv(ey);
