@@ -936,22 +936,30 @@ __device__ __forceinline__ int closure_finish(const DevScene& D, Ray& r, S* opt,
     return ended ? 1 : 0;
 }
 
+// Runs up to `budget` trials of a closure (0: to its end). Returns 1 with *h set when it finished.
+template <class S>
+__device__ __forceinline__ int closure_trials(const DevScene& D, S* opt, unsigned long long* cstats, int pidx, int kind,
+                                              CondState* cs, int budget, const Ray& r, float* wmul, Hist* h) {
+    const clr_scene_params& P = D.P;
+    const float COHERENT = fminf(fmaxf(D.coherent_f, 0.0f), 1.0f);
+    return conditional_interaction(
+        opt, h, pidx, D.qsca[pidx], D.qext[pidx], P.n_water, D.pn[pidx], D.pk[pidx], P.wavelength, P.rough_alpha,
+        D.prad[pidx], P.spheroid_aspect, P.orientation_model, P.orientation_kappa, P.max_particle_bounces, COHERENT,
+        D.phase_cdf, D.theta, D.phase_guide, D.nt, r.x, r.y, r.z, r.vx, r.vy, r.vz, P.rin, P.zmin, P.zmean,
+        P.free_surface_model,
+        P.vortex_delta_h, P.vortex_core_radius, kind == CK_GEOM ? P.conditional_retries - 1 : P.conditional_retries,
+        cstats, cs, budget, wmul, closure_trial_tag(r.ic));
+}
+
 // Runs (part of) a closure. Returns 0 when the iteration ended with the photon in the water, 1 when the
 // history ended, 2 when the closure continues (state in *cs; with budget 0 it always finishes).
 template <class S>
 __device__ __forceinline__ int closure_visit(const DevScene& D, Ray& r, S* opt, unsigned long long* cstats, int pidx,
                                              int kind, CondState* cs, int budget) {
-    const clr_scene_params& P = D.P;
-    const float COHERENT = fminf(fmaxf(D.coherent_f, 0.0f), 1.0f);
     Hist h;
-    const int done = conditional_interaction(
-        opt, &h, pidx, D.qsca[pidx], D.qext[pidx], P.n_water, D.pn[pidx], D.pk[pidx], P.wavelength, P.rough_alpha,
-        D.prad[pidx], P.spheroid_aspect, P.orientation_model, P.orientation_kappa, P.max_particle_bounces, COHERENT,
-        D.phase_cdf, D.theta, D.phase_guide, D.nt, r.x, r.y, r.z, r.vx, r.vy, r.vz, P.rin, P.zmin, P.zmean,
-        P.free_surface_model,
-        P.vortex_delta_h, P.vortex_core_radius, kind == CK_GEOM ? P.conditional_retries - 1 : P.conditional_retries,
-        cstats, cs, budget, (kind == CK_FLIGHT && weighted_run(D)) ? &r.w : nullptr, closure_trial_tag(r.ic));
-    if (!done) return 2;
+    if (!closure_trials(D, opt, cstats, pidx, kind, cs, budget, r,
+                        (kind == CK_FLIGHT && weighted_run(D)) ? &r.w : nullptr, &h))
+        return 2;
     return closure_finish(D, r, opt, pidx, kind, h);
 }
 
@@ -1040,6 +1048,40 @@ __device__ __forceinline__ int closure_visit_warp(const DevScene& D, Ray& r, Phi
     }
     if (!done) return 2;
     return closure_finish(D, r, opt, pidx, kind, h);
+}
+
+// The rest of a started closure across the warp (counter-based stream only; called by all 32 lanes with the
+// same photon): lane l runs trial cs->trial + l of every batch, one call of the serial closure's own function
+// with a budget of one trial, so every trial, the chosen one (the lowest that ends the closure) and every
+// counter are the serial loop's. `scratch` holds CLR_N_CONDITIONAL_STATS shared counters per lane. Worth its
+// up to 31 unused trials only once a closure has shown itself long.
+__device__ __forceinline__ int closure_rest_warp(const DevScene& D, Ray& r, PhiloxStream* opt,
+                                                 unsigned long long* cstats, int pidx, int kind, CondState* cs,
+                                                 unsigned long long* scratch) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int max_trials = kind == CK_GEOM ? D.P.conditional_retries - 1 : D.P.conditional_retries;
+    unsigned long long* mine = scratch + lane * CLR_N_CONDITIONAL_STATS;
+    Hist h;
+    while (true) {
+        for (int i = 0; i < CLR_N_CONDITIONAL_STATS; ++i) mine[i] = 0ull;
+        int fin = 0;
+        if (cs->trial + lane < max_trials) {
+            CondState one = {1, cs->trial + lane, cs->target};
+            fin = closure_trials(D, opt, mine, pidx, kind, &one, 1, r, (float*)nullptr, &h);
+        }
+        const unsigned term = __ballot_sync(FULL, fin != 0);
+        const int win = term ? __ffs(term) - 1 : 31;
+        if (lane <= win) {
+            for (int i = 0; i < CLR_N_CONDITIONAL_STATS; ++i)
+                if (mine[i]) atomicAdd(cstats + i, mine[i]);
+        }
+        if (term) {
+            h = shfl_hist(h, win);
+            return closure_finish(D, r, opt, pidx, kind, h);
+        }
+        cs->trial += 32;
+    }
 }
 
 template <class S>

@@ -71,6 +71,10 @@ constexpr int kCondInline = 8;
 constexpr int kCondBudget = 512;
 // trials per COND visit when a whole warp runs them (counter-based stream): 32 warp steps
 constexpr int kCondWarpBudget = 1024;
+// trials a lane runs on its own before the rest of its closure goes across the warp (diagnostic COND stage and
+// tail kernel, counter-based stream): most closures of a scattered target end in one or two, an absorbed
+// target of a weakly absorbing particle takes hundreds
+constexpr int kCondAlone = 12;
 
 template <class Mode>
 struct WavePool {
@@ -358,7 +362,8 @@ __device__ __forceinline__ int wave_stage_body(const WaveLaunch& w, const DevSce
             v = closure_visit(D, r, L.optics(), cstats, m.pidx, CK_GEOM, &cs, kCondInline);
         } else {
             cs.started = m.cond_started; cs.trial = m.cond_trial; cs.target = m.cond_target;
-            v = closure_visit(D, r, L.optics(), cstats, m.pidx, m.cond_kind, &cs, kCondBudget);
+            v = closure_visit(D, r, L.optics(), cstats, m.pidx, m.cond_kind, &cs,
+                              kCounterStream<typename Mode::Stream> ? kCondAlone : kCondBudget);
         }
         if (v == 2) {
             m.cond_started = cs.started; m.cond_trial = cs.trial; m.cond_target = cs.target;
@@ -491,20 +496,102 @@ __global__ void __launch_bounds__(kWaveThreads, 1) wave_cond_warp_kernel(WaveLau
     if (lane == 0 && sum) atomicAdd(&w.tallies[0].sched[WQ_COND], sum);
 }
 
+// The rest of the closure of the photon in `slot` across the warp (closure_rest_warp; called by all 32 lanes):
+// every lane reads the photon and ends with the same state, `owner` writes it back. Returns the photon's next
+// queue, the same in every lane.
+template <class Mode, bool kProv>
+__device__ __forceinline__ int cond_rest_visit(const WaveLaunch& w, const WavePool<Mode>& pool, uint32_t slot, int owner,
+                                               unsigned long long* scratch) {
+    Ray r = pool.ray[slot];
+    typename Mode::Lane L = pool.lane[slot];
+    const SlotMeta m = pool.meta[slot];
+    const DevScene& D = w.scenes[m.sid];
+    const int ic0 = r.ic, coh0 = r.wcoh, mor0 = r.wmorph;
+    const int per0 = r.pc.entry_reflections, pir0 = r.pc.internal_reflections;
+    const float vinx = r.vx, viny = r.vy, vinz = r.vz;
+    CondState cs;
+    cs.started = 1; cs.trial = m.cond_trial; cs.target = m.cond_target;
+    const int v = closure_rest_warp(D, r, L.optics(), w.tallies[m.sid].c.cstats, m.pidx, m.cond_kind, &cs, scratch);
+    __syncwarp();
+    if ((int)(threadIdx.x & 31) == owner) {
+        if constexpr (kProv) {
+            if (w.prov && r.ic == ic0) {  // as the per-lane stage body: survived, or ended by absorption
+                uint4 pv = w.prov[slot];
+                const int type = prov_type(r.wcoh - coh0, r.wmorph - mor0, r.pc.entry_reflections - per0,
+                                           r.pc.internal_reflections - pir0);
+                if (v == 0) prov_event(pv, r.ic, type, m.pidx, vinx, viny, vinz, r.vx, r.vy, r.vz);
+                else if (r.st == 5) prov_mark(pv, r.ic, type, m.pidx);
+                w.prov[slot] = pv;
+            }
+        }
+        pool.ray[slot] = r;
+        pool.lane[slot] = L;
+    }
+    __syncwarp();
+    return v ? WQ_FIN : WQ_FLIGHT;
+}
+
+// COND stage of diagnostic runs on the counter-based stream: each lane runs the first kCondAlone trials of its
+// photon's closure; the closures that go on are then finished one at a time across the warp. With all trials in
+// the lane (up to 512 per visit) the stage waited for single lanes: 2.3 active per instruction.
+template <class Mode>
+__global__ void __launch_bounds__(kWaveThreads, 1) wave_cond_diag_kernel(WaveLaunch w) {
+    const WaveWindow win = wave_window(w, WQ_COND);
+    if (win.n == 0) return;
+    __shared__ unsigned long long scratch[kWaveThreads * CLR_N_CONDITIONAL_STATS];
+    unsigned long long* mine = scratch + (threadIdx.x & ~31) * CLR_N_CONDITIONAL_STATS;
+    const WavePool<Mode> pool = wave_pool<Mode>(w);
+    const uint32_t* ring = wave_ring(w, WQ_COND);
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned long long done = 0;
+    for (unsigned base = wave_claim(w, WQ_COND); base < win.n; base = wave_claim(w, WQ_COND)) {
+        const unsigned i = base + lane;
+        const bool valid = i < win.n;
+        const uint32_t slot = valid ? ring[(win.head + i) & wave_mask(w)] : 0u;
+        int dest = -1;
+        if (valid) {
+            Ray r = pool.ray[slot];
+            typename Mode::Lane L = pool.lane[slot];
+            SlotMeta m = pool.meta[slot];
+            const DevScene& D = w.scenes[m.sid];
+            uint4 pvv;
+            uint4* pv = nullptr;
+            if (w.prov) { pvv = w.prov[slot]; pv = &pvv; }
+            dest = wave_stage_body<Mode, WQ_COND, true>(w, D, r, L, m, w.tallies[m.sid].c.cstats, pv);
+            if (pv) w.prov[slot] = pvv;
+            pool.ray[slot] = r;
+            pool.lane[slot] = L;
+            pool.meta[slot] = m;
+            done++;
+        }
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(FULL, dest == WQ_COND); todo; todo &= todo - 1u) {
+            const int owner = __ffs(todo) - 1;
+            const int next = cond_rest_visit<Mode, true>(w, pool, __shfl_sync(FULL, slot, owner), owner, mine);
+            if (lane == owner) dest = next;
+        }
+        wave_push(w, dest, slot);
+    }
+    const unsigned long long sum = __reduce_add_sync(FULL, (unsigned)done);
+    if (lane == 0 && sum) atomicAdd(&w.tallies[0].sched[WQ_COND], sum);
+}
+
 // The event-handler stage kernel: its provenance-counting variant when provenance is on.
 template <class Mode, int Q>
 const void* stage_fn(const void* prov) {
     return prov ? (const void*)wave_stage_kernel<Mode, Q, true> : (const void*)wave_stage_kernel<Mode, Q, false>;
 }
 
-// The COND stage kernel: warp-cooperative closures on the counter-based stream without diagnostics, else
-// the per-lane stage kernel.
+// The COND stage kernel: on the counter-based stream warp-cooperative closures (diagnostic runs: after the first
+// trials), on the xorshift streams, whose trials draw one after the other, the per-lane stage kernel.
 template <class Mode>
 const void* cond_fn(const WaveLaunch& w) {
     if constexpr (kCounterStream<typename Mode::Stream>) {
-        if (!w.prov && !w.light) return (const void*)wave_cond_warp_kernel<Mode>;
+        return (w.prov || w.light) ? (const void*)wave_cond_diag_kernel<Mode> : (const void*)wave_cond_warp_kernel<Mode>;
+    } else {
+        return stage_fn<Mode, WQ_COND>(w.prov);
     }
-    return stage_fn<Mode, WQ_COND>(w.prov);
 }
 
 // ---------------- FIN: detector scoring and tallies; the slot becomes free ----------------
