@@ -656,6 +656,12 @@ __device__ __forceinline__ int tail_visit(const WaveLaunch& w, int q, const DevS
 // Runs after the last pass, when every photon is drawn: the photons still queued (entries [snap, tail)
 // of every queue but FREE) are taken one per thread and carried through the same stage bodies, in the
 // same order, as the passes would carry them, then scored. Per-ray results are those of the passes.
+// Queue neighbours go to different warps (neighbours wait at the same surface and share its long traversals,
+// so a warp of them costs its lanes one after the other). The grid is one block of two warps per SM as long as
+// that takes every photon at once (no lane then waits for a second round), else a block per 64 photons: further
+// warps only add instruction-fetch stalls (no_instruction 2.2, 5.2 and 15.0 cycles per issue at 1, 2 and 6 warps
+// per SM; the dense weighted scene's tail 111, 94 and 120 ms). Tail of a 2e6-photon full-scene trace
+// 3.2 -> 1.0 ms, of 1e5 disc-beam photons 0.49 -> 0.30 ms, against queue order on n / 128 blocks of 128.
 template <class Mode, bool kRecord, bool kDiag>
 __global__ void __launch_bounds__(kTailThreads) wave_tail_kernel(WaveLaunch w) {
     __shared__ DetTable det;
@@ -668,7 +674,8 @@ __global__ void __launch_bounds__(kTailThreads) wave_tail_kernel(WaveLaunch w) {
     const unsigned total = first[CLR_WQ_COUNT];
     const WavePool<Mode> pool = wave_pool<Mode>(w);
     unsigned long long visits[CLR_WQ_COUNT] = {};
-    for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const unsigned warps = gridDim.x * (blockDim.x / 32), warp = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    for (unsigned idx = (threadIdx.x & 31) * warps + warp; idx < total; idx += 32u * warps) {
         int q = 1;
         while (idx >= first[q + 1]) ++q;
         const uint32_t slot = wave_ring(w, q)[(c->snap[q] + (idx - first[q])) & wave_mask(w)];
@@ -826,10 +833,12 @@ cudaError_t wave_run_t(const WaveLaunch& w, int num_sms, cudaStream_t st, long l
         if (live[1] != 0u) {
             // at most live[2] photons remain after the passes already queued: finish them in one launch
             const unsigned n = live[2];
-            const int blocks = (int)std::max(1u, std::min(n, 65536u * kTailThreads) / kTailThreads + 1);
+            const int threads = 64;  // of the kernel's kTailThreads
+            const unsigned spread = std::max((unsigned)num_sms, (n + threads - 1) / threads);
+            const int blocks = (int)std::min(spread, n / (threads / 32) + 1);
             if (w.tail_begin && (e = cudaEventRecord(w.tail_begin, st)) != cudaSuccess) return e;
-            if (w.light || w.prov) wave_tail_kernel<Mode, kRecord, true><<<blocks, kTailThreads, 0, st>>>(w);
-            else wave_tail_kernel<Mode, kRecord, false><<<blocks, kTailThreads, 0, st>>>(w);
+            if (w.light || w.prov) wave_tail_kernel<Mode, kRecord, true><<<blocks, threads, 0, st>>>(w);
+            else wave_tail_kernel<Mode, kRecord, false><<<blocks, threads, 0, st>>>(w);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
             if (w.tail_end && (e = cudaEventRecord(w.tail_end, st)) != cudaSuccess) return e;
             info->tail = 1;
