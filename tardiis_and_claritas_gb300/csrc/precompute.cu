@@ -18,6 +18,7 @@
 #include <cstdint>
 #include <cstring>
 #include <vector>
+#include <cooperative_groups.h>
 #include "kernels.h"
 
 namespace clr {
@@ -970,13 +971,13 @@ __device__ void merid_surface(int FSM, double r, double ZMEAN, double R, double 
     *zs = ZMEAN - hbar + Hinf * rr2 / (a2 + rr2);
     *hp = 2.0 * Hinf * a2 * rr / ((a2 + rr2) * (a2 + rr2));
 }
-// secondary-circulation velocity from the streamfunction psi = -2U r^2 (1-r^2/R^2)^2 eta(1-eta) (:4059-4073)
-__device__ void merid_velocity(double r, double z, double ZMIN, double ZMEAN, double R, int FSM, double DH, double CORE,
-                               double UPEAK, double* ur, double* uz) {
+// secondary-circulation velocity from the streamfunction psi = -2U r^2 (1-r^2/R^2)^2 eta(1-eta) (:4059-4073);
+// zs, hp: merid_surface at r
+__device__ void merid_velocity(double r, double z, double zs, double hp, double ZMIN, double R, int FSM, double DH,
+                               double CORE, double UPEAK, double* ur, double* uz) {
     *ur = 0.0; *uz = 0.0;
     if (!(UPEAK > 0.0) || !(R > 0.0) || !(DH > 0.0) || (FSM == 2 && !(CORE > 0.0))) return;
-    double rr = fmin(fmax(r, 0.0), R), R2 = R * R, rr2 = rr * rr, zs = ZMEAN, hp = 0.0;
-    merid_surface(FSM, rr, ZMEAN, R, DH, CORE, &zs, &hp);
+    double rr = fmin(fmax(r, 0.0), R), R2 = R * R, rr2 = rr * rr;
     double H = zs - ZMIN;
     if (!(H > 0.0)) return;
     double eta = (z - ZMIN) / H;
@@ -997,13 +998,8 @@ __device__ double merid_slip(int p, double r, double R, const double* WR, int NR
     long long b = (long long)p * (long long)NRAD;
     return (1.0 - t) * WR[b + j] + t * WR[b + j + 1];
 }
-// a point inside the liquid (:4084-4089)
-__device__ int merid_fluid(double r, double z, double ZMIN, double ZMEAN, double R, int FSM, double DH, double CORE) {
-    if (z < ZMIN) return 0;
-    double zs = ZMEAN, hp = 0.0;
-    merid_surface(FSM, r, ZMEAN, R, DH, CORE, &zs, &hp);
-    return z < zs;
-}
+// a point inside the liquid (:4084-4089); zs: merid_surface at its radius
+__device__ __forceinline__ int merid_fluid(double z, double zs, double ZMIN) { return z >= ZMIN && z < zs; }
 // the finite-Re drift-diffusion field at a cell centre (sediment_local_scale with model 2, :1560-1593),
 // which starts the iteration (:4100-4112)
 __device__ double merid_initial(int FSM, int p, const double* SA, const double* SB, const double* SN, const double* RL,
@@ -1058,12 +1054,19 @@ __device__ bool merid_grid_barrier(unsigned* count, unsigned* gen, unsigned nblo
     return ok_s != 0;
 }
 
+// A bin's rows are shared out over the CTAs of one thread-block cluster.
+__device__ __forceinline__ void cluster_sync() { cooperative_groups::this_cluster().sync(); }
+// the same shared-memory variable in the cluster's CTA `rank`
+__device__ __forceinline__ double* in_cluster(double* local, unsigned rank) {
+    return cooperative_groups::this_cluster().map_shared_rank(local, rank);
+}
+
 struct MeridArgs {
-    int n, NR, NZ, NRAD, FSM, max_it, check_every;
+    int n, NR, NZ, NRAD, FSM, max_it, check_every, cluster, mass_in_smem, coef_in_smem;
     double R, ZMIN, ZMEAN, ZGRIDMAX, DH, CORE, UPEAK, Dt, OMEGA, TOL;
     const double *sedA, *sedB, *sed_norm, *radial_log, *wr, *ws;
     double* grid;       // [n][NR][NZ]
-    double* coef;       // [n][5][NR*NZ]: AP, AE, AW, AN, AS
+    double* coef;       // [n][kMeridPlanes][NR*NZ]: work planes, see below
     double* grid_max;   // [n] largest value over the liquid cells
     double* residual;   // [2][n] residual of every bin at the last two checks
     unsigned* bar;      // [2] barrier count and generation (zero before the launch)
@@ -1073,160 +1076,287 @@ struct MeridArgs {
 };
 
 constexpr int kMeridThreads = 512;
+constexpr int kMeridMaxCluster = 8;
+// work planes per bin: AE, AW, AN, AS, AP and 1/AP of the relaxed cells in list order, the lists (cells of one
+// colour after the other, then the liquid cells in the reference's order; 2 x 32 bit per cell), the mass terms
+constexpr int kMeridPlanes = 8;
 
+// num / ap, correctly rounded, with rap = 1 / ap correctly rounded: one residual step on num * rap (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990). Three
+// FP64 operations on the relaxation's bounding pipe against the eight or more of a division. No operand here is
+// near the ends of the exponent range; an infinite or NaN num stays one.
+__device__ __forceinline__ double merid_div(double num, double ap, double rap) {
+    const double q = num * rap;
+    return fma(fma(-ap, q, num), rap, q);
+}
+
+// The solver is bound by the FP64 pipe (one warp instruction per 16 cycles per SM), so: only liquid cells of one
+// colour are listed, in full warps (a pass over the plane keeps half the lanes of every FP64 instruction idle);
+// the division costs three operations; and a bin's rows are spread over a cluster of CTAs so that n bins use
+// cluster x n SMs, neighbours' boundary rows written through distributed shared memory. 64 bins of 48x96 cells,
+// 1250 iterations: 78 ms with one CTA per bin over the whole plane. Values, order of every sum and stopping
+// iteration are unchanged.
 __global__ void __launch_bounds__(kMeridThreads) meridional_solve_kernel(MeridArgs a) {
     extern __shared__ __align__(16) unsigned char msm[];
-    const int NR = a.NR, NZ = a.NZ, plane = NR * NZ, p = blockIdx.x, tid = threadIdx.x;
-    double* G = reinterpret_cast<double*>(msm);
-    unsigned char* act = msm + (size_t)plane * 8;
+    const int NR = a.NR, NZ = a.NZ, plane = NR * NZ, tid = threadIdx.x, lane = tid & 31;
+    const unsigned CS = (unsigned)a.cluster, rank = cooperative_groups::this_cluster().block_rank();
+    const int p = blockIdx.x / a.cluster;
+    const int i0 = (int)((long long)NR * rank / CS), i1 = (int)((long long)NR * (rank + 1) / CS);  // this CTA's rows
+    // shared memory: the plane (every CTA holds all of it; its own rows and their two neighbours are current)
+    // with a zero row and cell on either side, the free surface at cell centres and faces, the liquid mask and,
+    // where it fits, the mass terms
+    double* const G0 = reinterpret_cast<double*>(msm);
+    const int pad = NZ + 1;
+    double* const G = G0 + pad;
+    double* const zsC = G0 + plane + 2 * pad;
+    double* const hpC = zsC + NR;
+    double* const zsF = hpC + NR;
+    double* const hpF = zsF + NR + 1;
+    double* const mass_sm = hpF + NR + 1;
+    unsigned char* const act = reinterpret_cast<unsigned char*>(mass_sm + (a.mass_in_smem ? plane : 0));
     __shared__ double red[kMeridThreads / 32];
-    __shared__ double scale_s;
-    __shared__ int bad_s;
+    __shared__ double from_rank[kMeridMaxCluster];  // rank 0: a value of every CTA
+    __shared__ double scale_s, go_s;                // written by rank 0 into every CTA
+    __shared__ int scan_s[3][kMeridThreads / 32];
     const double dr = a.R / (double)NR, dz = (a.ZGRIDMAX - a.ZMIN) / (double)NZ;
-    double* AP = a.coef + (size_t)p * 5 * plane;
-    double* AE = AP + plane;
-    double* AW = AE + plane;
-    double* AN = AW + plane;
-    double* AS = AN + plane;
+    double* const work = a.coef + (size_t)p * kMeridPlanes * plane;
+    const int b0 = i0 * NZ, b1 = i1 * NZ;
+    // the relaxed cells' coefficients and list: in shared memory where they fit (every cluster barrier would have
+    // the next sweep fetch them from L2 again), else in this CTA's part of the work planes
+    const size_t cells = (size_t)(b1 - b0), stride = a.coef_in_smem ? cells : (size_t)plane;
+    double* const AE = a.coef_in_smem ? reinterpret_cast<double*>(act + ((plane + 15) & ~15)) : work + b0;
+    double *const AW = AE + stride, *const AN = AW + stride, *const AS = AN + stride, *const AP = AS + stride,
+           *const RAP = AP + stride;
+    int* const lists = reinterpret_cast<int*>(work + 6 * (size_t)plane);
+    int* const relax_list = a.coef_in_smem ? reinterpret_cast<int*>(RAP + stride) : lists + b0;
+    int* const liquid_list = lists + plane + b0;
+    double* const mass_terms = a.mass_in_smem ? mass_sm : work + 7 * (size_t)plane;
+    // the free surface depends on the radius only
+    for (int i = tid; i <= NR; i += kMeridThreads) {
+        if (i < NR) merid_surface(a.FSM, ((double)i + 0.5) * dr, a.ZMEAN, a.R, a.DH, a.CORE, &zsC[i], &hpC[i]);
+        merid_surface(a.FSM, (double)i * dr, a.ZMEAN, a.R, a.DH, a.CORE, &zsF[i], &hpF[i]);
+    }
+    for (int c = tid; c < pad; c += kMeridThreads) { G0[c] = 0.0; G[plane + c] = 0.0; }
+    __syncthreads();
     // liquid cells (:4091-4098) and the starting field (:4100-4112)
     for (int c = tid; c < plane; c += kMeridThreads) {
         const int i = c / NZ, k = c - i * NZ;
-        const double r = ((double)i + 0.5) * dr, z = a.ZMIN + ((double)k + 0.5) * dz;
-        act[c] = (unsigned char)(merid_fluid(r, z, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE) ? 1 : 0);
+        const double zc = a.ZMIN + ((double)k + 0.5) * dz;
+        const int liquid = merid_fluid(zc, zsC[i], a.ZMIN);
+        act[c] = (unsigned char)liquid;
+        double g = 0.0;
+        if (liquid && i >= i0 - 1 && i <= i1) {
+            const float x = (float)(((double)i + 0.5) * dr), z = (float)zc;
+            g = merid_initial(a.FSM, p, a.sedA, a.sedB, a.sed_norm, a.radial_log, a.NRAD, x, z, (float)a.R, (float)a.ZMIN);
+        }
+        G[c] = g;
     }
     __syncthreads();
-    for (int c = tid; c < plane; c += kMeridThreads) {
-        const int i = c / NZ, k = c - i * NZ;
-        if (!act[c]) { G[c] = 0.0; continue; }
-        const float x = (float)(((double)i + 0.5) * dr), z = (float)(a.ZMIN + ((double)k + 0.5) * dz);
-        G[c] = merid_initial(a.FSM, p, a.sedA, a.sedB, a.sed_norm, a.radial_log, a.NRAD, x, z, (float)a.R,
-                             (float)a.ZMIN);
-    }
-    // upwind finite-volume coefficients (:4114-4159)
-    for (int c = tid; c < plane; c += kMeridThreads) {
-        const int i = c / NZ, k = c - i * NZ;
-        AP[c] = AE[c] = AW[c] = AN[c] = AS[c] = 0.0;
-        if (!act[c]) continue;
-        double rc = ((double)i + 0.5) * dr, zc = a.ZMIN + ((double)k + 0.5) * dz;
-        double rw = (double)i * dr, re = (double)(i + 1) * dr;
-        double Az = 0.5 * (re * re - rw * rw), ap = 0.0, ur = 0.0, uz = 0.0, V = 0.0, F = 0.0, diff = 0.0;
-        if (i + 1 < NR && act[(i + 1) * NZ + k] && merid_fluid(re, zc, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE)) {
-            merid_velocity(re, zc, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
-            V = ur + merid_slip(p, re, a.R, a.wr, a.NRAD); F = V * re * dz; diff = a.Dt * re * dz / dr;
-            AE[c] = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
-        }
-        if (i > 0 && act[(i - 1) * NZ + k] && merid_fluid(rw, zc, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE)) {
-            merid_velocity(rw, zc, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
-            V = ur + merid_slip(p, rw, a.R, a.wr, a.NRAD); F = -V * rw * dz; diff = a.Dt * rw * dz / dr;
-            AW[c] = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
-        }
-        double zf = zc + 0.5 * dz;
-        if (k + 1 < NZ && act[i * NZ + k + 1] && merid_fluid(rc, zf, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE)) {
-            merid_velocity(rc, zf, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
-            V = uz - a.ws[p]; F = V * Az; diff = a.Dt * Az / dz;
-            AN[c] = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
-        }
-        zf = zc - 0.5 * dz;
-        if (k > 0 && act[i * NZ + k - 1] && merid_fluid(rc, zf, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE)) {
-            merid_velocity(rc, zf, a.ZMIN, a.ZMEAN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
-            V = uz - a.ws[p]; F = -V * Az; diff = a.Dt * Az / dz;
-            AS[c] = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
-        }
-        AP[c] = ap;
-    }
+    // upwind finite-volume coefficients of this CTA's rows (:4114-4159), compacted: the cells the sweeps relax
+    // (liquid, with a positive diagonal), colour 0 then colour 1, and the liquid cells in plane order
+    int n_relax[2] = {0, 0}, n_liquid = 0, liquid_before = 0;
+    for (int c = tid; c < b0; c += kMeridThreads) liquid_before += act[c];
+    for (int o = 16; o > 0; o >>= 1) liquid_before += __shfl_xor_sync(0xffffffffu, liquid_before, o);
+    if (lane == 0) scan_s[0][tid >> 5] = liquid_before;
     __syncthreads();
-    // per-bin mass renormalisation (:4176-4187): the mass sum runs serially in the reference's order
-    auto normalize = [&]() {
-        if (tid == 0) {
-            double mass = 0.0;
-            for (int i = 0; i < NR; ++i) {
-                double rw = (double)i * dr, re = (double)(i + 1) * dr, vol = 0.5 * (re * re - rw * rw) * dz;
-                for (int k = 0; k < NZ; ++k) {
-                    const int c = i * NZ + k;
-                    if (act[c]) mass += G[c] * vol;
+    liquid_before = 0;
+    for (int w = 0; w < kMeridThreads / 32; ++w) liquid_before += scan_s[0][w];
+    for (int colour = 0; colour < 2; ++colour) {
+        for (int base = b0; base < b1; base += kMeridThreads) {
+            const int c = base + tid;
+            bool relax = false, liquid = false;
+            double ae = 0.0, aw = 0.0, an = 0.0, as = 0.0, ap = 0.0;
+            if (c < b1) {
+                const int i = c / NZ, k = c - i * NZ;
+                liquid = act[c] != 0;
+                if (liquid && ((i + k) & 1) == colour) {
+                    double rc = ((double)i + 0.5) * dr, zc = a.ZMIN + ((double)k + 0.5) * dz;
+                    double rw = (double)i * dr, re = (double)(i + 1) * dr;
+                    double Az = 0.5 * (re * re - rw * rw), ur = 0.0, uz = 0.0, V = 0.0, F = 0.0, diff = 0.0;
+                    if (i + 1 < NR && act[(i + 1) * NZ + k] && merid_fluid(zc, zsF[i + 1], a.ZMIN)) {
+                        merid_velocity(re, zc, zsF[i + 1], hpF[i + 1], a.ZMIN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
+                        V = ur + merid_slip(p, re, a.R, a.wr, a.NRAD); F = V * re * dz; diff = a.Dt * re * dz / dr;
+                        ae = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
+                    }
+                    if (i > 0 && act[(i - 1) * NZ + k] && merid_fluid(zc, zsF[i], a.ZMIN)) {
+                        merid_velocity(rw, zc, zsF[i], hpF[i], a.ZMIN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
+                        V = ur + merid_slip(p, rw, a.R, a.wr, a.NRAD); F = -V * rw * dz; diff = a.Dt * rw * dz / dr;
+                        aw = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
+                    }
+                    double zf = zc + 0.5 * dz;
+                    if (k + 1 < NZ && act[i * NZ + k + 1] && merid_fluid(zf, zsC[i], a.ZMIN)) {
+                        merid_velocity(rc, zf, zsC[i], hpC[i], a.ZMIN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
+                        V = uz - a.ws[p]; F = V * Az; diff = a.Dt * Az / dz;
+                        an = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
+                    }
+                    zf = zc - 0.5 * dz;
+                    if (k > 0 && act[i * NZ + k - 1] && merid_fluid(zf, zsC[i], a.ZMIN)) {
+                        merid_velocity(rc, zf, zsC[i], hpC[i], a.ZMIN, a.R, a.FSM, a.DH, a.CORE, a.UPEAK, &ur, &uz);
+                        V = uz - a.ws[p]; F = -V * Az; diff = a.Dt * Az / dz;
+                        as = diff + fmax(-F, 0.0); ap += diff + fmax(F, 0.0);
+                    }
+                    relax = ap > 0.0;
                 }
             }
+            const unsigned below = (1u << lane) - 1u;
+            const unsigned mr = __ballot_sync(0xffffffffu, relax), ml = __ballot_sync(0xffffffffu, liquid);
+            __syncthreads();
+            if (lane == 0) { scan_s[1][tid >> 5] = __popc(mr); scan_s[2][tid >> 5] = __popc(ml); }
+            __syncthreads();
+            int at_r = __popc(mr & below), at_l = __popc(ml & below), tot_r = 0, tot_l = 0;
+            for (int w = 0; w < kMeridThreads / 32; ++w) {
+                if (w < (tid >> 5)) { at_r += scan_s[1][w]; at_l += scan_s[2][w]; }
+                tot_r += scan_s[1][w]; tot_l += scan_s[2][w];
+            }
+            if (relax) {
+                const int q = (colour ? n_relax[0] : 0) + n_relax[colour] + at_r;
+                relax_list[q] = c;
+                AE[q] = ae; AW[q] = aw; AN[q] = an; AS[q] = as; AP[q] = ap; RAP[q] = 1.0 / ap;
+            }
+            n_relax[colour] += tot_r;
+            if (colour == 0) {
+                if (liquid) liquid_list[n_liquid + at_l] = c;
+                n_liquid += tot_l;
+            }
+        }
+    }
+    // this CTA's mass terms go to rank 0 (its shared memory, or the bin's global plane)
+    double* const mass_out = a.mass_in_smem ? in_cluster(mass_sm, 0u) : mass_terms;
+    cluster_sync();
+    int mass_count = 0;
+    for (int c = tid; c < plane; c += kMeridThreads) mass_count += act[c];
+    for (int o = 16; o > 0; o >>= 1) mass_count += __shfl_xor_sync(0xffffffffu, mass_count, o);
+    if (lane == 0) scan_s[0][tid >> 5] = mass_count;
+    __syncthreads();
+    mass_count = 0;
+    for (int w = 0; w < kMeridThreads / 32; ++w) mass_count += scan_s[0][w];
+    // per-bin mass renormalisation (:4176-4187): the terms in parallel, their sum in the reference's order
+    auto normalize = [&]() {
+        for (int j = tid; j < n_liquid; j += kMeridThreads) {
+            const int c = liquid_list[j], i = c / NZ;
+            double rw = (double)i * dr, re = (double)(i + 1) * dr, vol = 0.5 * (re * re - rw * rw) * dz;
+            mass_out[liquid_before + j] = G[c] * vol;
+        }
+        cluster_sync();
+        if (rank == 0 && tid < 32) {
+            const double mass = warp_serial_sum(mass_terms, mass_count, nullptr);
             double target = 0.5 * a.R * a.R * (a.ZMEAN - a.ZMIN);
-            bad_s = (!(mass > 0.0) || !(target > 0.0) || !isfinite(mass)) ? 1 : 0;
-            if (bad_s) atomicCAS(a.err, 0, 41);
-            scale_s = bad_s ? 1.0 : target / mass;
+            const bool bad = !(mass > 0.0) || !(target > 0.0) || !isfinite(mass);
+            if (bad && lane == 0) atomicCAS(a.err, 0, 41);
+            if (lane < (int)CS) *in_cluster(&scale_s, (unsigned)lane) = bad ? 1.0 : target / mass;
         }
-        __syncthreads();
-        if (!bad_s) {
-            const double sc = scale_s;
-            for (int c = tid; c < plane; c += kMeridThreads)
-                if (act[c]) G[c] *= sc;
-        }
-        __syncthreads();
+        cluster_sync();
+        // own rows and the neighbours' boundary rows (solid cells are zero)
+        const double sc = scale_s;
+        const int lo = max(0, i0 - 1) * NZ, hi = min(NR, i1 + 1) * NZ;
+        for (int c = lo + tid; c < hi; c += kMeridThreads) G[c] *= sc;
+        cluster_sync();
     };
+    double* const G_down = rank > 0 ? in_cluster(G, rank - 1) : nullptr;  // G in the CTAs of the rows below and above
+    double* const G_up = rank + 1 < CS ? in_cluster(G, rank + 1) : nullptr;
+    const double keep = 1.0 - a.OMEGA;
     // one colour of the red-black SOR sweep (:4161-4174)
-    auto relax = [&](int parity) {
-        for (int c = tid; c < plane; c += kMeridThreads) {
-            const int i = c / NZ, k = c - i * NZ;
-            if (!act[c] || ((i + k) & 1) != parity || !(AP[c] > 0.0)) continue;
-            double num = 0.0;
-            if (i + 1 < NR) num += AE[c] * G[(i + 1) * NZ + k];
-            if (i > 0) num += AW[c] * G[(i - 1) * NZ + k];
-            if (k + 1 < NZ) num += AN[c] * G[i * NZ + k + 1];
-            if (k > 0) num += AS[c] * G[i * NZ + k - 1];
-            double target = num / AP[c], old = G[c], nv = (1.0 - a.OMEGA) * old + a.OMEGA * target;
-            if (!isfinite(nv) || nv < 1e-14) nv = 1e-14;
+    auto relax = [&](int colour) {
+        const int q0 = colour ? n_relax[0] : 0, q1 = q0 + n_relax[colour];
+        for (int q = q0 + tid; q < q1; q += kMeridThreads) {
+            const int c = relax_list[q];
+            double num = AE[q] * G[c + NZ];
+            num += AW[q] * G[c - NZ];
+            num += AN[q] * G[c + 1];
+            num += AS[q] * G[c - 1];
+            double nv = keep * G[c] + a.OMEGA * merid_div(num, AP[q], RAP[q]);
+            // nv not finite, or nv < 1e-14: on the bits, which the FP64 pipe need not see
+            const long long bits = __double_as_longlong(nv);
+            if ((bits & 0x7ff0000000000000LL) == 0x7ff0000000000000LL || bits < __double_as_longlong(1e-14)) nv = 1e-14;
             G[c] = nv;
+            if (c < b0 + NZ && G_down) G_down[c] = nv;
+            if (c >= b1 - NZ && G_up) G_up[c] = nv;
         }
+        cluster_sync();
+    };
+    // the largest of one value per CTA over the cluster, in every thread of rank 0
+    auto cluster_max = [&](double m) -> double {
+        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) red[tid >> 5] = m;
         __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < kMeridThreads / 32; ++w) m = fmax(m, red[w]);
+            *in_cluster(&from_rank[rank], 0u) = m;
+        }
+        cluster_sync();
+        double all = 0.0;
+        if (rank == 0)
+            for (unsigned q = 0; q < CS; ++q) all = fmax(all, from_rank[q]);
+        return all;
+    };
+    // the decision of rank 0's first thread in every CTA of the cluster
+    auto agree = [&](double v) -> double {
+        if (rank == 0 && tid == 0)
+            for (unsigned q = 0; q < CS; ++q) *in_cluster(&go_s, q) = v;
+        cluster_sync();
+        const double r = go_s;
+        cluster_sync();
+        return r;
     };
     // largest relative residual of the bin (:4189-4197)
     auto residual = [&]() -> double {
         double mr = 0.0;
-        for (int c = tid; c < plane; c += kMeridThreads) {
-            const int i = c / NZ, k = c - i * NZ;
-            if (!act[c] || !(AP[c] > 0.0)) continue;
-            double num = 0.0;
-            if (i + 1 < NR) num += AE[c] * G[(i + 1) * NZ + k];
-            if (i > 0) num += AW[c] * G[(i - 1) * NZ + k];
-            if (k + 1 < NZ) num += AN[c] * G[i * NZ + k + 1];
-            if (k > 0) num += AS[c] * G[i * NZ + k - 1];
-            double den = fmax(fabs(AP[c] * G[c]), 1e-30), q = fabs(AP[c] * G[c] - num) / den;
-            if (q > mr) mr = q;
+        for (int q = tid; q < n_relax[0] + n_relax[1]; q += kMeridThreads) {
+            const int c = relax_list[q];
+            double num = AE[q] * G[c + NZ];
+            num += AW[q] * G[c - NZ];
+            num += AN[q] * G[c + 1];
+            num += AS[q] * G[c - 1];
+            const double ap = AP[q];
+            double den = fmax(fabs(ap * G[c]), 1e-30), r = fabs(ap * G[c] - num) / den;
+            if (r > mr) mr = r;
         }
-        for (int o = 16; o > 0; o >>= 1) mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, o));
-        if ((tid & 31) == 0) red[tid >> 5] = mr;
-        __syncthreads();
-        double m = 0.0;
-        for (int w = 0; w < kMeridThreads / 32; ++w) m = fmax(m, red[w]);
-        __syncthreads();
-        return m;
+        return cluster_max(mr);
     };
     normalize();
     const int min_it = a.max_it < 1000 ? a.max_it : 1000;
     int done = 0, last_checked = 0, checks = 0;
     double worst = 0.0;
-    bool stop = false;
-    // the initial normalisation is checked before the first sweep (:6561-6575)
-    if (!merid_grid_barrier(a.bar, a.bar + 1, gridDim.x, a.err)) stop = true;
-    if (!stop && *(volatile int*)a.err) stop = true;
-    for (int it = 1; it <= a.max_it && !stop; ++it) {
+    // the bins meet through rank 0 of each cluster; every CTA of a cluster follows its decision
+    // (0 go on, 1 stop before the first sweep, 2 converged, 3 give up)
+    double verdict = 0.0;
+    if (rank == 0) {
+        // the initial normalisation is checked before the first sweep (:6561-6575)
+        if (!merid_grid_barrier(a.bar, a.bar + 1, (unsigned)a.n, a.err) || *(volatile int*)a.err) verdict = 1.0;
+    }
+    verdict = agree(verdict);
+    for (int it = 1; it <= a.max_it && verdict == 0.0; ++it) {
         relax(0);
         relax(1);
         if (it % 20 == 0) normalize();
         if (it % a.check_every == 0 || it == a.max_it) {
             normalize();
             const double r = residual();
-            double* slot = a.residual + (size_t)(checks & 1) * a.n;
-            if (tid == 0) slot[p] = r;
-            if (!merid_grid_barrier(a.bar, a.bar + 1, gridDim.x, a.err)) break;
-            worst = 0.0;
-            for (int q = 0; q < a.n; ++q) worst = fmax(worst, ((volatile double*)slot)[q]);
-            last_checked = it;
-            ++checks;
-            if (*(volatile int*)a.err) break;
-            if (it >= min_it && worst <= a.TOL) { done = it; break; }
+            if (rank == 0) {
+                double* slot = a.residual + (size_t)(checks & 1) * a.n;
+                if (tid == 0) slot[p] = r;
+                if (!merid_grid_barrier(a.bar, a.bar + 1, (unsigned)a.n, a.err)) {
+                    verdict = 3.0;
+                } else {
+                    worst = 0.0;
+                    for (int q = 0; q < a.n; ++q) worst = fmax(worst, ((volatile double*)slot)[q]);
+                    last_checked = it;
+                    ++checks;
+                    if (*(volatile int*)a.err) verdict = 3.0;
+                    else if (it >= min_it && worst <= a.TOL) { done = it; verdict = 2.0; }
+                }
+            }
+            verdict = agree(verdict);
         }
     }
     if (done == 0) done = last_checked ? last_checked : a.max_it;
-    if (p == 0 && tid == 0) { *a.iterations = done; *a.max_residual = worst; }
+    if (p == 0 && rank == 0 && tid == 0) { *a.iterations = done; *a.max_residual = worst; }
+    double mx = 0.0;
+    for (int c = b0 + tid; c < b1; c += kMeridThreads)
+        if (act[c] && G[c] > mx) mx = G[c];
+    __syncthreads();
     // extend each column above the free surface with its highest liquid value (:4199-4205)
-    for (int i = tid; i < NR; i += kMeridThreads) {
+    for (int i = i0 + tid; i < i1; i += kMeridThreads) {
         int top = -1;
         for (int k = NZ - 1; k >= 0; --k)
             if (act[i * NZ + k]) { top = k; break; }
@@ -1235,22 +1365,13 @@ __global__ void __launch_bounds__(kMeridThreads) meridional_solve_kernel(MeridAr
         for (int k = top + 1; k < NZ; ++k) G[i * NZ + k] = q;
     }
     __syncthreads();
-    double mx = 0.0;
-    for (int c = tid; c < plane; c += kMeridThreads) {
-        a.grid[(size_t)p * plane + c] = G[c];
-        if (act[c] && G[c] > mx) mx = G[c];
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0) red[tid >> 5] = mx;
-    __syncthreads();
-    if (tid == 0) {
-        double m = 0.0;
-        for (int w = 0; w < kMeridThreads / 32; ++w) m = fmax(m, red[w]);
-        a.grid_max[p] = m;  // the majorant kernel takes 1 where this is not positive (:4207-4209)
-    }
+    for (int c = b0 + tid; c < b1; c += kMeridThreads) a.grid[(size_t)p * plane + c] = G[c];
+    mx = cluster_max(mx);
+    if (rank == 0 && tid == 0) a.grid_max[p] = mx;  // the majorant kernel takes 1 where this is not positive (:4207-4209)
+    cluster_sync();  // no CTA leaves while another may still write to it
 }
 
-size_t meridional_coef_doubles(int n, int nr, int nz) { return (size_t)n * 5 * nr * nz; }
+size_t meridional_coef_doubles(int n, int nr, int nz) { return (size_t)n * kMeridPlanes * nr * nz; }
 
 cudaError_t enqueue_meridional_solve(ParticleBuffers& pb, const clr_scene_params& sp, const clr_sediment_spec& ss,
                                      cudaStream_t st) {
@@ -1264,14 +1385,40 @@ cudaError_t enqueue_meridional_solve(ParticleBuffers& pb, const clr_scene_params
     a.ws = pb.sed_ws; a.grid = pb.sed_grid; a.coef = pb.merid_coef; a.grid_max = pb.grid_max;
     a.residual = pb.merid_residual; a.bar = pb.merid_bar; a.err = pb.err; a.iterations = pb.merid_stats;
     a.max_residual = reinterpret_cast<double*>(pb.merid_residual + 2 * (size_t)pb.n);
-    const size_t smem = (size_t)a.NR * a.NZ * 9;
-    cudaError_t e = cudaFuncSetAttribute(meridional_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    const size_t plane = (size_t)a.NR * a.NZ, limit = 226 * 1024;
+    const size_t base = (plane + 2 * ((size_t)a.NZ + 1) + 4 * (size_t)a.NR + 2) * sizeof(double) + ((plane + 15) & ~(size_t)15);
+    cudaError_t e = cudaFuncSetAttribute(meridional_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(pb.merid_bar, 0, 2 * sizeof(unsigned), st)) != cudaSuccess) return e;
-    void* args[] = {&a};
-    return cudaLaunchCooperativeKernel((const void*)meridional_solve_kernel, dim3(a.n), dim3(kMeridThreads), args,
-                                       smem, st);
+    // the largest cluster with every bin's cluster resident at once (the bins wait for one another at the checks)
+    // and at least four rows per CTA
+    for (a.cluster = kMeridMaxCluster;; a.cluster /= 2) {
+        // beside the planes, as they fit: a CTA's coefficients (52 bytes per cell of its rows), rank 0's mass terms
+        const size_t rows = ((size_t)a.NR + a.cluster - 1) / a.cluster, coef = rows * a.NZ * (6 * sizeof(double) + sizeof(int));
+        size_t smem = base;
+        a.coef_in_smem = smem + coef <= limit ? 1 : 0;
+        if (a.coef_in_smem) smem += coef;
+        a.mass_in_smem = smem + plane * sizeof(double) <= limit ? 1 : 0;
+        if (a.mass_in_smem) smem += plane * sizeof(double);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)a.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeCooperative;
+        at[1].val.cooperative = 1;
+        cfg.gridDim = dim3((unsigned)(a.n * a.cluster)); cfg.blockDim = dim3(kMeridThreads);
+        cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
+        if (a.cluster > 1) {
+            if (a.NR < 4 * a.cluster) continue;
+            int fit = 0;
+            if (cudaOccupancyMaxActiveClusters(&fit, meridional_solve_kernel, &cfg) != cudaSuccess || fit < a.n) {
+                (void)cudaGetLastError();
+                continue;
+            }
+        }
+        cfg.numAttrs = 2;
+        return cudaLaunchKernelEx(&cfg, meridional_solve_kernel, a);
+    }
 }
 
 // Upper bound of the orders the Mie kernel needs for n bins: the largest nmx = max(nstop, |m x|) + 128 of
