@@ -131,15 +131,23 @@ __host__ __device__ constexpr uint64_t smem_desc(uint32_t addr, uint32_t lbo, ui
 constexpr int kM = 128, kN = 256, kKC = 64;  // rows per tile, output width, K per shared-memory stage
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both
 // K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) |
-                            ((uint32_t)(kM >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc_of(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
+}
+constexpr uint32_t kIdesc = idesc_of(kN);
 
-constexpr int kGemmThreads = 128;               // one warpgroup: warp w reads TMEM lanes 32w..32w+31
+// The training products are small (2048 x 256 x 256), so a launch's time is a tile's own chain: operands in, MMAs,
+// epilogue. A CTA takes 64 of the 256 output columns (64 CTAs for 2048 rows instead of 16), brings its whole
+// K = 256 in with asynchronous copies before the first MMA (four stages of 64), and eight warps share the
+// epilogue, 32 columns each. With 128 x 256 tiles, plain loads two stages deep and four warps a layer took 52 us.
+constexpr int kNT = 64;                         // output columns per CTA
+constexpr int kStages = 4;
+constexpr int kGemmThreads = 256;               // warp w reads TMEM lanes 32 (w % 4) .., columns 32 (w / 4) ..
 constexpr int kStageA = kM * kKC * 2;           // 16 KB
-constexpr int kStageB = kN * kKC * 2;           // 32 KB
-constexpr int kGemmSmem = 2 * (kStageA + kStageB) + 64;  // two stages, barriers, TMEM address
+constexpr int kStageB = kNT * kKC * 2;          // 8 KB
+constexpr int kGemmSmem = kStages * (kStageA + kStageB) + 64;  // stages, barriers, TMEM address
 
-enum Epi : int { EPI_STORE_F32 = 0, EPI_FWD = 1, EPI_BWD = 2, EPI_ATOMIC_F32 = 3, EPI_INFER = 4 };
+enum Epi : int { EPI_STORE_F32 = 0, EPI_FWD = 1, EPI_BWD = 2, EPI_ADD_F32 = 3 };
 
 struct GemmArgs {
     const bf16* A;           // [M][lda], K contiguous
@@ -147,25 +155,32 @@ struct GemmArgs {
     const bf16* B;           // [256][ldb], K contiguous
     long long ldb;
     int M, K, k_split;       // K and k_split multiples of 64; CTA y takes K columns [y*k_split, +k_split)
-    const float* bias;       // [256] (EPI_FWD, EPI_INFER)
+    const float* bias;       // [256] (EPI_FWD)
     const float* zin;        // [M][256] saved pre-activations (EPI_BWD)
-    float* out_f32;          // [M][ldo]: result (STORE, ATOMIC) or pre-activation z (FWD)
+    float* out_f32;          // [M][ldo]: result (STORE, ADD) or pre-activation z (FWD)
     long long ldo;
-    bf16* out_bf16;          // [M][256]: silu(z) (FWD, INFER) or dz (BWD)
+    bf16* out_bf16;          // [M][256]: silu(z) (FWD) or dz (BWD)
     bf16* out_bf16_t;        // [256][ldt]: transposed copy (FWD, BWD)
     long long ldt;
     int* err;
 };
+constexpr int kGemmBatch = 3;  // products of one launch (the weight gradients of the three hidden layers)
+struct GemmBatch { GemmArgs g[kGemmBatch]; };
 
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
+    const int bytes = valid ? 16 : 0;  // 0: the 16 bytes are zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
 // One K chunk (64 columns) of `rows` rows into the core-matrix layout: element (r, k) at
-// (r / 8) * 1024 + (k / 8) * 128 + (r % 8) * 16 + (k % 8) * 2 bytes. Rows at or past `valid` read as zero.
+// (r / 8) * 1024 + (k / 8) * 128 + (r % 8) * 16 + (k % 8) * 2 bytes. Rows at or past `valid` read as zero. Two
+// neighbouring lanes take 32 contiguous bytes of a row, 16 lanes apart rows: whole sectors, no bank conflicts.
 __device__ __forceinline__ void load_chunk(unsigned char* dst, const bf16* src, long long ld, int row0, int rows,
                                            int valid, int k0) {
     for (int q = threadIdx.x; q < rows * 8; q += kGemmThreads) {
-        const int r = q >> 3, kc = q & 7;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (row0 + r < valid) v = *reinterpret_cast<const uint4*>(src + (long long)(row0 + r) * ld + k0 + kc * 8);
-        *reinterpret_cast<uint4*>(dst + (r >> 3) * 1024 + kc * 128 + (r & 7) * 16) = v;
+        const int kc = (q & 1) | ((q >> 4) & 6), r = ((q >> 1) & 15) | ((q >> 7) << 4);
+        const bool ok = row0 + r < valid;
+        cp_async16(dst + (r >> 3) * 1024 + kc * 128 + (r & 7) * 16,
+                   src + (long long)(ok ? row0 + r : 0) * ld + k0 + kc * 8, ok);
     }
 }
 
@@ -176,23 +191,32 @@ __device__ __forceinline__ float dsilu_f(float z) {
 }
 
 template <int EPI>
-__global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(GemmArgs g) {
+__global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch batch) {
     extern __shared__ __align__(1024) unsigned char sm[];
+    const GemmArgs& g = batch.g[blockIdx.z / (kN / kNT)];
     unsigned char* const stA0 = sm;
-    unsigned char* const stB0 = sm + 2 * kStageA;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + 2 * (kStageA + kStageB));  // [2]
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
+    unsigned char* const stB0 = sm + kStages * kStageA;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kStages * (kStageA + kStageB));  // [kStages]
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + kStages);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * kM;
+    const int m0 = blockIdx.x * kM, n0 = (blockIdx.z % (kN / kNT)) * kNT;
     const int kb = blockIdx.y * g.k_split;
     const int ke = min(g.K, kb + g.k_split);
     const int nc = ke > kb ? (ke - kb) / kKC : 0;
+    auto load = [&](int c) {
+        const int st = c % kStages;
+        load_chunk(stA0 + st * kStageA, g.A, g.lda, m0, kM, g.M, kb + c * kKC);
+        load_chunk(stB0 + st * kStageB, g.B, g.ldb, n0, kNT, kN, kb + c * kKC);
+    };
+    for (int c = 0; c < kStages - 1; ++c) {
+        if (c < nc) load(c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int i = 0; i < kStages; ++i) mbar_init(&bar[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(tslot, 256);
+    if (warp == 0) tmem_alloc(tslot, kNT);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -200,49 +224,56 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(GemmArgs g) 
     bool ok = true;
     int issued = 0;  // chunks whose MMAs were issued
     for (int c = 0; c < nc; ++c) {
-        const int s = c & 1;
-        // the MMAs of chunk c-2 read this stage: wait for their commit
-        if (c >= 2) ok = mbar_wait(&bar[s], ((c - 2) >> 1) & 1, g.err, 1);
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-        load_chunk(stA0 + s * kStageA, g.A, g.lda, m0, kM, g.M, kb + c * kKC);
-        load_chunk(stB0 + s * kStageB, g.B, g.ldb, 0, kN, kN, kb + c * kKC);
+        const int pc = c + kStages - 1;
+        if (pc < nc) {
+            // the MMAs of chunk pc - kStages read this stage: wait for their commit
+            if (pc >= kStages) {
+                ok = mbar_wait(&bar[pc % kStages], ((pc - kStages) / kStages) & 1, g.err, 1);
+                if (!__syncthreads_and(ok)) { ok = false; break; }
+            }
+            load(pc);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
         fence_proxy_async();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t a0 = smem_u32(stA0 + s * kStageA), b0 = smem_u32(stB0 + s * kStageB);
+            const uint32_t a0 = smem_u32(stA0 + (c % kStages) * kStageA), b0 = smem_u32(stB0 + (c % kStages) * kStageB);
 #pragma unroll
             for (int kk = 0; kk < kKC / 16; ++kk)
-                mma_bf16(tmem, smem_desc(a0 + kk * 256, 128, 1024), smem_desc(b0 + kk * 256, 128, 1024), kIdesc,
+                mma_bf16(tmem, smem_desc(a0 + kk * 256, 128, 1024), smem_desc(b0 + kk * 256, 128, 1024), idesc_of(kNT),
                          (c > 0 || kk > 0) ? 1u : 0u);
-            mma_commit(&bar[s]);
+            mma_commit(&bar[c % kStages]);
         }
         issued = c + 1;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (issued > 0) {
         // the last commit covers every MMA issued before it; after a time-out wait once more (bounded)
         // so no MMA still writes the accumulator when it is released
-        const bool done = mbar_wait(&bar[(issued - 1) & 1], ((issued - 1) >> 1) & 1, g.err, 2);
+        const bool done = mbar_wait(&bar[(issued - 1) % kStages], ((issued - 1) / kStages) & 1, g.err, 2);
         ok = ok && done;
     }
     ok = __syncthreads_and(ok);
     tc_fence_after();
     if (ok && issued > 0) {
-        const int m = m0 + 32 * warp + lane;
-        const bool row_ok = m < g.M;
+        const int m = m0 + 32 * (warp & 3) + lane, j0 = n0 + 32 * (warp >> 2);
         float v[32];
-        for (int j0 = 0; j0 < kN; j0 += 32) {
-            tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)j0, v);
-            if (!row_ok) continue;
+        tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * (warp >> 2)), v);
+        if (m < g.M) {
             if constexpr (EPI == EPI_STORE_F32) {
                 float4* o = reinterpret_cast<float4*>(g.out_f32 + (long long)m * g.ldo + j0);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            } else if constexpr (EPI == EPI_ATOMIC_F32) {
+            } else if constexpr (EPI == EPI_ADD_F32) {
                 float* o = g.out_f32 + (long long)m * g.ldo + j0;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) atomicAdd(o + i, v[i]);
-            } else if constexpr (EPI == EPI_FWD || EPI == EPI_INFER) {
+                for (int i = 0; i < 8; ++i)
+                    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o + 4 * i), "f"(v[4 * i]),
+                                 "f"(v[4 * i + 1]), "f"(v[4 * i + 2]), "f"(v[4 * i + 3])
+                                 : "memory");
+            } else if constexpr (EPI == EPI_FWD) {
                 __align__(16) bf16 hb[32];
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
@@ -253,13 +284,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(GemmArgs g) 
                 uint4* ho = reinterpret_cast<uint4*>(g.out_bf16 + (long long)m * kN + j0);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) ho[i] = reinterpret_cast<const uint4*>(hb)[i];
-                if constexpr (EPI == EPI_FWD) {
-                    float4* zo = reinterpret_cast<float4*>(g.out_f32 + (long long)m * kN + j0);
+                float4* zo = reinterpret_cast<float4*>(g.out_f32 + (long long)m * kN + j0);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) zo[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                for (int i = 0; i < 8; ++i) zo[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) g.out_bf16_t[(long long)(j0 + i) * g.ldt + m] = hb[i];
-                }
+                for (int i = 0; i < 32; ++i) g.out_bf16_t[(long long)(j0 + i) * g.ldt + m] = hb[i];
             } else {  // EPI_BWD: dz = dh * silu'(z)
                 const float4* zi = reinterpret_cast<const float4*>(g.zin + (long long)m * kN + j0);
                 __align__(16) bf16 db[32];
@@ -283,7 +312,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(GemmArgs g) 
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, 256);
+        tmem_dealloc(tmem, kNT);
     }
 }
 
@@ -291,8 +320,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(GemmArgs g) 
 // stream capture).
 static cudaError_t set_gemm_attributes() {
     const void* fns[] = {(const void*)umma_gemm_kernel<EPI_STORE_F32>, (const void*)umma_gemm_kernel<EPI_FWD>,
-                         (const void*)umma_gemm_kernel<EPI_BWD>, (const void*)umma_gemm_kernel<EPI_ATOMIC_F32>,
-                         (const void*)umma_gemm_kernel<EPI_INFER>};
+                         (const void*)umma_gemm_kernel<EPI_BWD>, (const void*)umma_gemm_kernel<EPI_ADD_F32>};
     for (const void* f : fns) {
         cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
         if (e != cudaSuccess) return e;
@@ -300,133 +328,199 @@ static cudaError_t set_gemm_attributes() {
     return cudaSuccess;
 }
 
+// `count` products of one shape in one launch.
 template <int EPI>
-static cudaError_t launch_gemm(const GemmArgs& g, int grid_y, cudaStream_t st) {
-    dim3 grid((g.M + kM - 1) / kM, grid_y);
-    umma_gemm_kernel<EPI><<<grid, kGemmThreads, kGemmSmem, st>>>(g);
+static cudaError_t launch_gemm(const GemmBatch& b, int count, int grid_y, cudaStream_t st) {
+    dim3 grid((b.g[0].M + kM - 1) / kM, grid_y, count * (kN / kNT));
+    umma_gemm_kernel<EPI><<<grid, kGemmThreads, kGemmSmem, st>>>(b);
     return cudaGetLastError();
 }
 
 // ---------------- CUDA-core kernels: thin layers, loss, gradients, optimizer ----------------
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
-// rows of the batch by index (training) or copied (inference: idx null)
-// (w: per-output loss weights of the rows, nullable)
-__global__ void gather_kernel(const float* __restrict__ x, const float* __restrict__ t, const float* __restrict__ w,
-                              const int32_t* __restrict__ idx, long long row0, int n, float* xb, float* tb,
-                              float* wb) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const long long src = idx ? (long long)idx[row0 + r] : row0 + r;
-#pragma unroll
-    for (int i = 0; i < kIn; ++i) xb[r * kIn + i] = bfr(x[src * kIn + i]);
-    if (t && tb)
-#pragma unroll
-        for (int i = 0; i < kOut; ++i) tb[r * kOut + i] = t[src * kOut + i];
-    if (w && wb)
-#pragma unroll
-        for (int i = 0; i < kOut; ++i) wb[r * kOut + i] = w[src * kOut + i];
-}
+// Inputs of the training steps of one call, in device memory (so the captured step serves every call):
+// the caller's rows and the step about to run.
+struct StepArgs {
+    const float *x, *t, *w;  // [rows][6], [rows][3], loss weights [rows][3] or null
+    const int32_t* idx;      // row of each position, or null (position i is row i)
+    int step;                // steps begun in this call; the head kernel counts it up
+};
+constexpr int kThinRows = 16;  // batch rows per block of the thin layers
 
-// layer 1 (6 -> 256): one thread per (row, unit)
-__global__ void layer1_kernel(const float* __restrict__ xb, int n, const bf16* __restrict__ w1,
-                              const float* __restrict__ b1, float* z1, bf16* h1, bf16* h1t, long long ldt) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)n * kHid) return;
-    const int r = (int)(t / kHid), j = (int)(t % kHid);
-    float z = b1[j];
-#pragma unroll
-    for (int i = 0; i < kIn; ++i) z = fmaf(xb[r * kIn + i], __bfloat162float(w1[j * kIn + i]), z);
-    const bf16 h = __float2bfloat16(silu_f(z));
-    h1[(long long)r * kHid + j] = h;
-    if (z1) z1[(long long)r * kHid + j] = z;
-    if (h1t) h1t[(long long)j * ldt + r] = h;
-}
+__device__ __forceinline__ uint4 pack8(const bf16* v) { return *reinterpret_cast<const uint4*>(v); }
 
-// Output layer (256 -> 3), one warp per row; with targets also the loss L = sum w (y - t)^2 / (3 n) (w = 1
-// without weights), dy = dL/dy and the gradient through the output layer into the last hidden layer
-// (dz4 = (dy . W5) * silu'(z4)).
-__global__ void head_kernel(const bf16* __restrict__ h4, const float* __restrict__ z4, int n,
-                            const bf16* __restrict__ w5, const float* __restrict__ b5, const float* __restrict__ tb,
-                            const float* __restrict__ wb, float* y, float* dy, bf16* dz4, bf16* dz4t, long long ldt,
-                            float* loss_sum) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const int r = warp;
-    float hv[8], acc[kOut] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) hv[i] = __bfloat162float(h4[(long long)r * kHid + lane * 8 + i]);
-#pragma unroll
-    for (int k = 0; k < kOut; ++k)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[k] = fmaf(hv[i], __bfloat162float(w5[k * kHid + lane * 8 + i]), acc[k]);
-#pragma unroll
-    for (int k = 0; k < kOut; ++k)
-        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-    float yv[kOut];
-#pragma unroll
-    for (int k = 0; k < kOut; ++k) yv[k] = acc[k] + b5[k];
-    if (y && lane == 0)
-#pragma unroll
-        for (int k = 0; k < kOut; ++k) y[r * kOut + k] = yv[k];
-    if (!tb) return;
-    const float scale = 2.0f / (3.0f * (float)n);
-    float d[kOut], l = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kOut; ++k) {
-        const float e = yv[k] - tb[r * kOut + k];
-        const float we = wb ? wb[r * kOut + k] * e : e;
-        d[k] = scale * we;
-        l += we * e;
+// Gather and layer 1 (6 -> 256): 16 rows per block, thread j one unit. Rows of z and h are stored across the
+// threads, and each thread's 16 activations of its unit as two 16-byte stores of the transposed copy.
+__global__ void __launch_bounds__(kHid) layer1_kernel(const StepArgs* __restrict__ a, int n, const bf16* __restrict__ w1,
+                                                      const float* __restrict__ b1, float* xb, float* tb, float* wb,
+                                                      float* z1, bf16* h1, bf16* h1t, long long ldt) {
+    __shared__ float xs[kThinRows * kIn];
+    const int r0 = blockIdx.x * kThinRows, j = threadIdx.x;
+    const long long row0 = (long long)a->step * n;
+    if (j < kThinRows * kIn) {
+        const int r = j / kIn, i = j % kIn;
+        const long long src = a->idx ? (long long)a->idx[row0 + r0 + r] : row0 + r0 + r;
+        const float v = bfr(a->x[src * kIn + i]);
+        xs[j] = v;
+        xb[r0 * kIn + j] = v;
+    } else if (j >= 128 && j < 128 + kThinRows * kOut) {
+        const int q = j - 128, r = q / kOut, i = q % kOut;
+        const long long src = a->idx ? (long long)a->idx[row0 + r0 + r] : row0 + r0 + r;
+        tb[r0 * kOut + q] = a->t[src * kOut + i];
+        wb[r0 * kOut + q] = a->w ? a->w[src * kOut + i] : 1.0f;
     }
-    if (lane == 0) {
+    float w[kIn];
 #pragma unroll
-        for (int k = 0; k < kOut; ++k) dy[r * kOut + k] = d[k];
+    for (int i = 0; i < kIn; ++i) w[i] = __bfloat162float(w1[j * kIn + i]);
+    const float b = b1[j];
+    __syncthreads();
+    __align__(16) bf16 hv[kThinRows];
+#pragma unroll
+    for (int r = 0; r < kThinRows; ++r) {
+        float z = b;
+#pragma unroll
+        for (int i = 0; i < kIn; ++i) z = fmaf(xs[r * kIn + i], w[i], z);
+        hv[r] = __float2bfloat16(silu_f(z));
+        h1[(long long)(r0 + r) * kHid + j] = hv[r];
+        z1[(long long)(r0 + r) * kHid + j] = z;
+    }
+    uint4* o = reinterpret_cast<uint4*>(h1t + (long long)j * ldt + r0);
+    o[0] = pack8(hv);
+    o[1] = pack8(hv + 8);
+}
+
+// Output layer (256 -> 3), one warp per row (16 rows per block): the loss L = sum w (y - t)^2 / (3 n), dy = dL/dy
+// and the gradient through the output layer into the last hidden layer (dz4 = (dy . W5) * silu'(z4)); the
+// transposed copy goes through shared memory, the loss is added once per block.
+__global__ void __launch_bounds__(256) head_kernel(StepArgs* a, const bf16* __restrict__ h4, const float* __restrict__ z4,
+                                                   int n, const bf16* __restrict__ w5, const float* __restrict__ b5,
+                                                   const float* __restrict__ tb, const float* __restrict__ wb, float* dy,
+                                                   bf16* dz4, bf16* dz4t, long long ldt, float* loss_sum) {
+    __shared__ bf16 tile[kThinRows][kHid + 8];
+    __shared__ float block_loss[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = blockIdx.x * kThinRows;
+    if (blockIdx.x == 0 && threadIdx.x == 0) a->step += 1;
+    float wv[kOut][8], lsum = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kOut; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) wv[k][i] = __bfloat162float(w5[k * kHid + lane * 8 + i]);
+    const float scale = 2.0f / (3.0f * (float)n);
+#pragma unroll
+    for (int q = 0; q < kThinRows / 8; ++q) {
+        const int lr = warp + 8 * q, r = r0 + lr;
+        float hv[8], acc[kOut] = {0.0f, 0.0f, 0.0f};
+        const uint4 hq = *reinterpret_cast<const uint4*>(h4 + (long long)r * kHid + lane * 8);
+        const float4 za = *reinterpret_cast<const float4*>(z4 + (long long)r * kHid + lane * 8),
+                     zb = *reinterpret_cast<const float4*>(z4 + (long long)r * kHid + lane * 8 + 4);
+        const float zv[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) hv[i] = __bfloat162float(reinterpret_cast<const bf16*>(&hq)[i]);
+#pragma unroll
+        for (int k = 0; k < kOut; ++k) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[k] = fmaf(hv[i], wv[k][i], acc[k]);
+            for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        }
+        float d[kOut], l = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kOut; ++k) {
+            const float e = acc[k] + b5[k] - tb[r * kOut + k];
+            const float we = wb[r * kOut + k] * e;
+            d[k] = scale * we;
+            l += we * e;
+        }
+        lsum += l;
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < kOut; ++k) dy[r * kOut + k] = d[k];
+        }
+        __align__(16) bf16 dv[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float g = 0.0f;
+#pragma unroll
+            for (int k = 0; k < kOut; ++k) g = fmaf(d[k], wv[k][i], g);
+            dv[i] = __float2bfloat16(g * dsilu_f(zv[i]));
+        }
+        *reinterpret_cast<uint4*>(dz4 + (long long)r * kHid + lane * 8) = pack8(dv);
+        *reinterpret_cast<uint4*>(&tile[lr][lane * 8]) = pack8(dv);
+    }
+    if (lane == 0) block_loss[warp] = lsum;
+    __syncthreads();
+    __align__(16) bf16 col[kThinRows];
+#pragma unroll
+    for (int r = 0; r < kThinRows; ++r) col[r] = tile[r][threadIdx.x];
+    uint4* o = reinterpret_cast<uint4*>(dz4t + (long long)threadIdx.x * ldt + r0);
+    o[0] = pack8(col);
+    o[1] = pack8(col + 8);
+    if (threadIdx.x == 0) {
+        float l = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) l += block_loss[w];
         atomicAdd(loss_sum, l);
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int j = lane * 8 + i;
-        float g = 0.0f;
-#pragma unroll
-        for (int k = 0; k < kOut; ++k) g = fmaf(d[k], __bfloat162float(w5[k * kHid + j]), g);
-        const bf16 v = __float2bfloat16(g * dsilu_f(z4[(long long)r * kHid + j]));
-        dz4[(long long)r * kHid + j] = v;
-        dz4t[(long long)j * ldt + r] = v;
-    }
 }
 
-// Small gradient reductions over the batch, one thread per output, rows split over blockIdx.y:
-//   db_l[j] = sum_r dz_l[r][j] (l = 1..4, from the transposed copies), dW1[j][i] = sum_r dz1[r][j] x[r][i],
-//   dW5[k][j] = sum_r dy[r][k] h4[r][j], db5[k] = sum_r dy[r][k].
-__global__ void small_grads_kernel(const bf16* const* __restrict__ dzt, long long ldt, const float* __restrict__ xb,
-                                   const float* __restrict__ dy, const bf16* __restrict__ h4, int n, int rows_per,
-                                   float* grads) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r0 = blockIdx.y * rows_per, r1 = min(n, r0 + rows_per);
-    constexpr int kBias = 4 * kHid, kW1 = kHid * kIn, kW5 = kOut * kHid;
-    if (t < kBias) {
-        const int l = t / kHid, j = t % kHid;
-        const bf16* row = dzt[l] + (long long)j * ldt;
-        float s = 0.0f;
-        for (int r = r0; r < r1; ++r) s += __bfloat162float(row[r]);
-        atomicAdd(grads + off_b(l + 1) + j, s);
-    } else if (t < kBias + kW1) {
-        const int q = t - kBias, j = q / kIn, i = q % kIn;
-        const bf16* row = dzt[0] + (long long)j * ldt;
-        float s = 0.0f;
-        for (int r = r0; r < r1; ++r) s = fmaf(__bfloat162float(row[r]), xb[r * kIn + i], s);
-        atomicAdd(grads + kOffW1 + q, s);
-    } else if (t < kBias + kW1 + kW5) {
-        const int q = t - kBias - kW1, k = q / kHid, j = q % kHid;
-        float s = 0.0f;
-        for (int r = r0; r < r1; ++r) s = fmaf(dy[r * kOut + k], __bfloat162float(h4[(long long)r * kHid + j]), s);
-        atomicAdd(grads + kOffW5 + q, s);
-    } else if (t < kBias + kW1 + kW5 + kOut) {
-        const int k = t - kBias - kW1 - kW5;
-        float s = 0.0f;
-        for (int r = r0; r < r1; ++r) s += dy[r * kOut + k];
-        atomicAdd(grads + kOffB5 + k, s);
+// Small gradient reductions over the batch, a thread per unit and 256 rows, each row after the other; a unit's rows
+// are contiguous in the transposed copies and come in 16 bytes at a time, 64 rows ahead; the rows' inputs and
+// output gradients are staged in shared memory (a thread that loads them row by row waits for memory at each):
+//   db_l[j] = sum_r dz_l[r][j] (l = 1..4), with it for l = 1 dW1[j][i] = sum_r dz1[r][j] x[r][i];
+//   dW5[k][j] = sum_r dy[r][k] h4[r][j]; and one thread for db5[k] = sum_r dy[r][k].
+constexpr int kSmallUnits = 5 * kHid + 1;
+constexpr int kSmallRows = 256;
+constexpr int kSmallThreads = 64;
+__global__ void __launch_bounds__(kSmallThreads) small_grads_kernel(const bf16* const* __restrict__ dzt,
+                                                                    const bf16* __restrict__ h4t, long long ldt,
+                                                                    const float* __restrict__ xb,
+                                                                    const float* __restrict__ dy, int n, float* grads) {
+    __shared__ float xs[kSmallRows * kIn], ds[kSmallRows * kOut];
+    const int r0 = blockIdx.y * kSmallRows, rows = min(n - r0, kSmallRows);  // a multiple of 128
+    const int unit = blockIdx.x * kSmallThreads + threadIdx.x;
+    const int what = unit / kHid, j = unit % kHid;  // 0..3: layer what + 1; 4: output weights; 5: output bias
+    if (what == 0)
+        for (int i = threadIdx.x; i < rows * kIn; i += kSmallThreads) xs[i] = xb[r0 * kIn + i];
+    if (what >= 4)
+        for (int i = threadIdx.x; i < rows * kOut; i += kSmallThreads) ds[i] = dy[r0 * kOut + i];
+    __syncthreads();
+    if (unit >= kSmallUnits) return;
+    const uint4* row = reinterpret_cast<const uint4*>((what < 4 ? dzt[what] : h4t) + (long long)j * ldt + r0);
+    float s[1 + kIn] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (what == 5) {
+#pragma unroll 8
+        for (int r = 0; r < rows; ++r)
+#pragma unroll
+            for (int k = 0; k < kOut; ++k) s[k] += ds[r * kOut + k];
+    } else {
+        for (int r = 0; r < rows; r += 64) {
+            uint4 q[8];
+#pragma unroll
+            for (int h = 0; h < 8; ++h) q[h] = row[r / 8 + h];
+#pragma unroll
+            for (int h = 0; h < 64; ++h) {
+                const float v = __bfloat162float(reinterpret_cast<const bf16*>(q)[h]);
+                if (what == 4) {
+#pragma unroll
+                    for (int k = 0; k < kOut; ++k) s[k] = fmaf(ds[(r + h) * kOut + k], v, s[k]);
+                } else {
+                    s[kIn] += v;
+                    if (what == 0) {
+#pragma unroll
+                        for (int i = 0; i < kIn; ++i) s[i] = fmaf(v, xs[(r + h) * kIn + i], s[i]);
+                    }
+                }
+            }
+        }
+    }
+    if (what < 4) {
+        atomicAdd(grads + off_b(what + 1) + j, s[kIn]);
+        if (what == 0)
+#pragma unroll
+            for (int i = 0; i < kIn; ++i) atomicAdd(grads + kOffW1 + j * kIn + i, s[i]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kOut; ++k) atomicAdd(grads + (what == 4 ? kOffW5 + k * kHid + j : kOffB5 + k), s[k]);
     }
 }
 
@@ -442,41 +536,48 @@ struct PackArgs {
 __host__ __device__ __forceinline__ int img_idx(int r, int k) {
     return ((r >> 3) * 4096 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2) >> 1;
 }
-__device__ __forceinline__ void pack_one(const PackArgs& pa, long long p, float v) {
+__device__ __forceinline__ void pack_one(const PackArgs& pa, int p, float v) {
     const bf16 b = __float2bfloat16(v);
-    for (int l = 1; l <= 5; ++l) {
-        const int nin = (l == 1) ? kIn : kHid;
-        const int nout = (l == 5) ? kOut : kHid;
-        const long long o = p - off_w(l);
-        if (o >= 0 && o < (long long)nin * nout) {
-            pa.w[l][o] = b;
-            const int out = (int)(o / nin), in = (int)(o % nin);
-            if (pa.wt[l]) pa.wt[l][(long long)in * nout + out] = b;
-            if (pa.wp[l]) {
-                if (l == 1)  // 256 x 16 image (K = 16): 8-row groups 256 bytes apart
-                    pa.wp[1][((out >> 3) * 256 + (in >> 3) * 128 + (out & 7) * 16 + (in & 7) * 2) >> 1] = b;
-                else
-                    pa.wp[l][img_idx(out, in)] = b;  // 256 x 256, or 16 x 256 for W5 (rows 3..15 stay zero)
-            }
-        }
+    if (p < (int)kOffB1) {
+        const int out = p / kIn, in = p % kIn;
+        pa.w[1][p] = b;
+        // 256 x 16 image (K = 16): 8-row groups 256 bytes apart
+        pa.wp[1][((out >> 3) * 256 + (in >> 3) * 128 + (out & 7) * 16 + (in & 7) * 2) >> 1] = b;
+    } else if (p < (int)kOffW5) {
+        // layers 2..4: weights and biases repeat every 256 x 256 + 256 parameters
+        constexpr int kStep = (int)(kOffW3 - kOffW2);
+        const int l = 2 + (p - (int)kOffW2) / kStep, o = (p - (int)kOffW2) % kStep;
+        if (p < (int)kOffW2 || o >= kHid * kHid) return;  // a bias
+        const int out = o / kHid, in = o % kHid;
+        pa.w[l][o] = b;
+        pa.wt[l][in * kHid + out] = b;
+        pa.wp[l][img_idx(out, in)] = b;
+    } else if (p < (int)kOffB5) {
+        const int o = p - (int)kOffW5;
+        pa.w[5][o] = b;
+        pa.wp[5][img_idx(o / kHid, o % kHid)] = b;  // 16 x 256, rows 3..15 stay zero
     }
 }
+static_assert(kOffW4 - kOffW3 == kOffW3 - kOffW2 && kOffW5 - kOffW4 == kOffW3 - kOffW2, "hidden layers are equally spaced");
 __global__ void pack_kernel(const float* __restrict__ params, PackArgs pa) {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < kParams) pack_one(pa, p, params[p]);
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < (int)kParams) pack_one(pa, p, params[p]);
 }
 
-// Adam (bias-corrected) on every parameter, then the gradient is cleared and the BF16 copies refreshed.
-__global__ void adam_kernel(float* params, float* grads, float* m1, float* m2, float lr, float b1, float b2,
-                            float eps, float c1, float c2, PackArgs pa) {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kParams) return;
+// Adam (bias-corrected) on every parameter, then the gradient is cleared and the BF16 copies refreshed. hp: per
+// step of the call the learning rate and the two bias corrections.
+__global__ void adam_kernel(float* params, float* grads, float* m1, float* m2, const StepArgs* __restrict__ step,
+                            const float4* __restrict__ hp, PackArgs pa) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= (int)kParams) return;
+    const float4 h = hp[step->step - 1];
+    const float lr = h.x, c1 = h.y, c2 = h.z;
     const float g = grads[p];
-    const float a = b1 * m1[p] + (1.0f - b1) * g;
-    const float b = b2 * m2[p] + (1.0f - b2) * g * g;
+    const float a = 0.9f * m1[p] + 0.1f * g;
+    const float b = 0.999f * m2[p] + 0.001f * g * g;
     m1[p] = a;
     m2[p] = b;
-    const float v = params[p] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+    const float v = params[p] - lr * (a / c1) / (sqrtf(b / c2) + 1e-8f);
     params[p] = v;
     grads[p] = 0.0f;
     pack_one(pa, p, v);
@@ -717,22 +818,21 @@ struct clr_mlp {
     bf16* dz[5] = {};          // [cap][256] gradients at the pre-activations
     bf16* dzt[5] = {};         // [256][cap]
     const bf16** d_dzt = nullptr;  // device array of dzt[1..4]
-    float *xb = nullptr, *tb = nullptr, *dy = nullptr, *y = nullptr, *loss = nullptr;
+    float *xb = nullptr, *tb = nullptr, *dy = nullptr, *loss = nullptr;
     float* wb = nullptr;          // [cap][3] loss weights of the batch rows
     const float* d_w = nullptr;   // the caller's loss weights (clr_mlp_set_loss_weights), or null
     int* d_err = nullptr;
     long long steps = 0;
     float last_ms = 0.0f;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // one captured training step per batch size
+    cudaStream_t side = nullptr;  // the small gradient reductions
+    cudaEvent_t fork = nullptr, join = nullptr;
+    // the captured training step of batch size step_n; its inputs are read from device memory
     cudaGraphExec_t step_exec = nullptr;
     int step_n = 0;
-    const float* step_x = nullptr;
-    const float* step_t = nullptr;
-    const int32_t* step_idx = nullptr;
-    const float* step_w = nullptr;
-    long long* d_row0 = nullptr;  // device copy of the batch's first index position (graph input)
-    float* d_lr = nullptr;        // device scalars of the captured Adam step: lr, c1, c2
+    StepArgs* d_step = nullptr;
+    float4* d_hp = nullptr;  // lr, c1, c2 of every step of the call
+    long long hp_cap = 0;
 };
 
 static int mfail(clr_mlp* m, int code, const char* msg) {
@@ -754,56 +854,58 @@ static cudaError_t malloc_tracked(clr_mlp* m, void** p, size_t bytes) {
     return e;
 }
 
-// Forward pass of n rows (n <= cap) already gathered into xb. With `train` the pre-activations and
-// transposed activations are kept for the backward pass.
-static cudaError_t forward_rows(clr_mlp* m, int n, bool train, cudaStream_t st) {
-    const int thr = 256;
-    layer1_kernel<<<(int)(((long long)n * kHid + thr - 1) / thr), thr, 0, st>>>(
-        m->xb, n, m->pa.w[1], m->params + kOffB1, train ? m->z[1] : nullptr, m->h[1], train ? m->ht[1] : nullptr,
-        m->cap);
+// Forward pass of the n rows (a multiple of 128, n <= cap) that d_step names; pre-activations and transposed
+// activations are kept for the backward pass.
+static cudaError_t forward_rows(clr_mlp* m, int n, cudaStream_t st) {
+    layer1_kernel<<<n / kThinRows, kHid, 0, st>>>(m->d_step, n, m->pa.w[1], m->params + kOffB1, m->xb, m->tb, m->wb,
+                                                  m->z[1], m->h[1], m->ht[1], m->cap);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     for (int l = 2; l <= 4; ++l) {
-        GemmArgs g{};
+        GemmBatch b{};
+        GemmArgs& g = b.g[0];
         g.A = m->h[l - 1]; g.lda = kHid; g.B = m->pa.w[l]; g.ldb = kHid;
         g.M = n; g.K = kHid; g.k_split = kHid;
         g.bias = m->params + off_b(l);
         g.out_f32 = m->z[l]; g.ldo = kHid; g.out_bf16 = m->h[l]; g.out_bf16_t = m->ht[l]; g.ldt = m->cap;
         g.err = m->d_err;
-        e = train ? launch_gemm<EPI_FWD>(g, 1, st) : launch_gemm<EPI_INFER>(g, 1, st);
-        if (e != cudaSuccess) return e;
+        if ((e = launch_gemm<EPI_FWD>(b, 1, 1, st)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
 // Backward pass of the n rows of the last forward (targets in tb): gradients accumulate into grads.
 static cudaError_t backward_rows(clr_mlp* m, int n, cudaStream_t st) {
-    head_kernel<<<(n * 32 + 255) / 256, 256, 0, st>>>(m->h[4], m->z[4], n, m->pa.w[5], m->params + kOffB5, m->tb,
-                                                      m->d_w ? m->wb : nullptr,
-                                                      m->y, m->dy, m->dz[4], m->dzt[4], m->cap, m->loss);
+    head_kernel<<<n / kThinRows, 256, 0, st>>>(m->d_step, m->h[4], m->z[4], n, m->pa.w[5], m->params + kOffB5, m->tb,
+                                               m->wb, m->dy, m->dz[4], m->dzt[4], m->cap, m->loss);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     for (int l = 4; l >= 2; --l) {  // dz_{l-1} = (dz_l . W_l) * silu'(z_{l-1})
-        GemmArgs g{};
+        GemmBatch b{};
+        GemmArgs& g = b.g[0];
         g.A = m->dz[l]; g.lda = kHid; g.B = m->pa.wt[l]; g.ldb = kHid;
         g.M = n; g.K = kHid; g.k_split = kHid;
         g.zin = m->z[l - 1]; g.out_bf16 = m->dz[l - 1]; g.out_bf16_t = m->dzt[l - 1]; g.ldt = m->cap;
         g.err = m->d_err;
-        if ((e = launch_gemm<EPI_BWD>(g, 1, st)) != cudaSuccess) return e;
+        if ((e = launch_gemm<EPI_BWD>(b, 1, 1, st)) != cudaSuccess) return e;
     }
+    // the small reductions run beside the weight gradients
+    if ((e = cudaEventRecord(m->fork, st)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(m->side, m->fork, 0)) != cudaSuccess) return e;
+    small_grads_kernel<<<dim3((kSmallUnits + kSmallThreads - 1) / kSmallThreads, (n + kSmallRows - 1) / kSmallRows),
+                         kSmallThreads, 0, m->side>>>(m->d_dzt, m->ht[4], m->cap, m->xb, m->dy, n, m->grads);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(m->join, m->side)) != cudaSuccess) return e;
     const int ksplit = 512;
-    for (int l = 2; l <= 4; ++l) {  // dW_l = dz_l^T . h_{l-1}, split over the batch
-        GemmArgs g{};
+    GemmBatch b{};
+    for (int l = 2; l <= 4; ++l) {  // dW_l = dz_l^T . h_{l-1}, split over the batch, the three layers in one launch
+        GemmArgs& g = b.g[l - 2];
         g.A = m->dzt[l]; g.lda = m->cap; g.B = m->ht[l - 1]; g.ldb = m->cap;
         g.M = kHid; g.K = n; g.k_split = ksplit;
         g.out_f32 = m->grads + off_w(l); g.ldo = kHid; g.err = m->d_err;
-        if ((e = launch_gemm<EPI_ATOMIC_F32>(g, (n + ksplit - 1) / ksplit, st)) != cudaSuccess) return e;
     }
-    const int rows_per = 256;
-    const int outs = 4 * kHid + kHid * kIn + kOut * kHid + kOut;
-    dim3 grid((outs + 255) / 256, (n + rows_per - 1) / rows_per);
-    small_grads_kernel<<<grid, 256, 0, st>>>(m->d_dzt, m->cap, m->xb, m->dy, m->h[4], n, rows_per, m->grads);
-    return cudaGetLastError();
+    if ((e = launch_gemm<EPI_ADD_F32>(b, kGemmBatch, (n + ksplit - 1) / ksplit, st)) != cudaSuccess) return e;
+    return cudaStreamWaitEvent(st, m->join, 0);
 }
 
 static int check_dev(clr_mlp* m) {
@@ -832,6 +934,9 @@ int clr_mlp_create(clr_mlp** out, int device, int max_batch, uint64_t seed) {
     MCU(cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, device));
     MCU(cudaEventCreate(&m->ev0));
     MCU(cudaEventCreate(&m->ev1));
+    MCU(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
+    MCU(cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming));
+    MCU(cudaEventCreateWithFlags(&m->join, cudaEventDisableTiming));
     auto F = [&](float** p, size_t cnt) { return malloc_tracked(m, (void**)p, cnt * sizeof(float)); };
     auto H = [&](bf16** p, size_t cnt) { return malloc_tracked(m, (void**)p, cnt * sizeof(bf16)); };
     MCU(F(&m->params, kParams)); MCU(F(&m->grads, kParams)); MCU(F(&m->m1, kParams)); MCU(F(&m->m2, kParams));
@@ -853,11 +958,10 @@ int clr_mlp_create(clr_mlp** out, int device, int max_batch, uint64_t seed) {
         MCU(H(&m->dz[l], act)); MCU(H(&m->dzt[l], act));
     }
     MCU(F(&m->xb, (size_t)m->cap * kIn)); MCU(F(&m->tb, (size_t)m->cap * kOut)); MCU(F(&m->wb, (size_t)m->cap * kOut));
-    MCU(F(&m->dy, (size_t)m->cap * kOut)); MCU(F(&m->y, (size_t)m->cap * kOut)); MCU(F(&m->loss, 4));
+    MCU(F(&m->dy, (size_t)m->cap * kOut)); MCU(F(&m->loss, 4));
     MCU(malloc_tracked(m, (void**)&m->d_err, sizeof(int)));
     MCU(malloc_tracked(m, (void**)&m->d_dzt, 4 * sizeof(bf16*)));
-    MCU(malloc_tracked(m, (void**)&m->d_row0, sizeof(long long)));
-    MCU(F(&m->d_lr, 4));
+    MCU(malloc_tracked(m, (void**)&m->d_step, sizeof(StepArgs)));
     const bf16* dzt[4] = {m->dzt[1], m->dzt[2], m->dzt[3], m->dzt[4]};
     MCU(cudaMemcpy(m->d_dzt, dzt, sizeof dzt, cudaMemcpyHostToDevice));
     MCU(cudaMemset(m->d_err, 0, sizeof(int)));
@@ -887,8 +991,12 @@ int clr_mlp_destroy(clr_mlp* m) {
     if (m->stream) cudaStreamSynchronize(m->stream);
     if (m->step_exec) cudaGraphExecDestroy(m->step_exec);
     for (void* p : m->allocs) cudaFree(p);
+    cudaFree(m->d_hp);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
+    if (m->fork) cudaEventDestroy(m->fork);
+    if (m->join) cudaEventDestroy(m->join);
+    if (m->side) cudaStreamDestroy(m->side);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return CLR_OK;
@@ -947,9 +1055,9 @@ int clr_mlp_gradients(clr_mlp* m, const float* d_x, const float* d_t, int64_t n,
     cudaStream_t st = m->stream;
     MCU(cudaMemsetAsync(m->grads, 0, kParams * sizeof(float), st));
     MCU(cudaMemsetAsync(m->loss, 0, sizeof(float), st));
-    gather_kernel<<<((int)n + 255) / 256, 256, 0, st>>>(d_x, d_t, m->d_w, nullptr, 0, (int)n, m->xb, m->tb, m->wb);
-    MCU(cudaGetLastError());
-    MCU(forward_rows(m, (int)n, true, st));
+    const StepArgs args = {d_x, d_t, m->d_w, nullptr, 0};
+    MCU(cudaMemcpyAsync(m->d_step, &args, sizeof args, cudaMemcpyHostToDevice, st));
+    MCU(forward_rows(m, (int)n, st));
     MCU(backward_rows(m, (int)n, st));
     float ls = 0.0f;
     MCU(cudaMemcpyAsync(&ls, m->loss, sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -963,44 +1071,9 @@ int clr_mlp_gradients(clr_mlp* m, const float* d_x, const float* d_t, int64_t n,
 
 }  // extern "C"
 
-// Gathers batch rows by index, with the batch start read from device memory so the captured step
-// serves every batch of an epoch.
-__global__ void gather_dev_kernel(const float* __restrict__ x, const float* __restrict__ t,
-                                  const float* __restrict__ w, const int32_t* __restrict__ idx,
-                                  const long long* __restrict__ row0, int n, float* xb, float* tb, float* wb) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const long long src = (long long)idx[*row0 + r];
-#pragma unroll
-    for (int i = 0; i < kIn; ++i) xb[r * kIn + i] = bfr(x[src * kIn + i]);
-#pragma unroll
-    for (int i = 0; i < kOut; ++i) tb[r * kOut + i] = t[src * kOut + i];
-    if (w)
-#pragma unroll
-        for (int i = 0; i < kOut; ++i) wb[r * kOut + i] = w[src * kOut + i];
-}
-
-__global__ void adam_dev_kernel(float* params, float* grads, float* m1, float* m2, const float* __restrict__ hp,
-                                PackArgs pa) {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kParams) return;
-    const float lr = hp[0], c1 = hp[1], c2 = hp[2];
-    const float g = grads[p];
-    const float a = 0.9f * m1[p] + 0.1f * g;
-    const float b = 0.999f * m2[p] + 0.001f * g * g;
-    m1[p] = a;
-    m2[p] = b;
-    const float v = params[p] - lr * (a / c1) / (sqrtf(b / c2) + 1e-8f);
-    params[p] = v;
-    grads[p] = 0.0f;
-    pack_one(pa, p, v);
-}
-
 // One training step (gather, forward, backward, Adam) captured as a graph for batch size n.
-static int build_step_graph(clr_mlp* m, const float* d_x, const float* d_t, const int32_t* d_idx, int n) {
-    if (m->step_exec && m->step_n == n && m->step_x == d_x && m->step_t == d_t && m->step_idx == d_idx &&
-        m->step_w == m->d_w)
-        return CLR_OK;
+static int build_step_graph(clr_mlp* m, int n) {
+    if (m->step_exec && m->step_n == n) return CLR_OK;
     if (m->step_exec) {
         cudaGraphExecDestroy(m->step_exec);
         m->step_exec = nullptr;
@@ -1008,13 +1081,11 @@ static int build_step_graph(clr_mlp* m, const float* d_x, const float* d_t, cons
     cudaStream_t st = m->stream;
     cudaGraph_t graph;
     MCU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    gather_dev_kernel<<<(n + 255) / 256, 256, 0, st>>>(d_x, d_t, m->d_w, d_idx, m->d_row0, n, m->xb, m->tb, m->wb);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = forward_rows(m, n, true, st);
+    cudaError_t e = forward_rows(m, n, st);
     if (e == cudaSuccess) e = backward_rows(m, n, st);
     if (e == cudaSuccess) {
-        adam_dev_kernel<<<(int)((kParams + 255) / 256), 256, 0, st>>>(m->params, m->grads, m->m1, m->m2, m->d_lr,
-                                                                       m->pa);
+        adam_kernel<<<(int)((kParams + 255) / 256), 256, 0, st>>>(m->params, m->grads, m->m1, m->m2, m->d_step, m->d_hp,
+                                                                  m->pa);
         e = cudaGetLastError();
     }
     cudaError_t e2 = cudaStreamEndCapture(st, &graph);
@@ -1023,7 +1094,7 @@ static int build_step_graph(clr_mlp* m, const float* d_x, const float* d_t, cons
     e = cudaGraphInstantiate(&m->step_exec, graph, 0);
     cudaGraphDestroy(graph);
     MCU(e);
-    m->step_n = n; m->step_x = d_x; m->step_t = d_t; m->step_idx = d_idx; m->step_w = m->d_w;
+    m->step_n = n;
     return CLR_OK;
 }
 
@@ -1033,21 +1104,32 @@ extern "C" int clr_mlp_train(clr_mlp* m, const float* d_x, const float* d_t, con
         return mfail(m, CLR_ERR_INVALID_ARGUMENT,
                      "clr_mlp_train: batch must be a multiple of 128 up to max_batch, and at most n_index");
     MCU(cudaSetDevice(m->device));
-    int rc = build_step_graph(m, d_x, d_t, d_index, batch);
-    if (rc != CLR_OK) return rc;
     cudaStream_t st = m->stream;
-    MCU(cudaMemsetAsync(m->loss, 0, sizeof(float), st));
     const long long steps = n_index / batch;
-    MCU(cudaEventRecord(m->ev0, st));
-    for (long long s = 0; s < steps; ++s) {
-        const long long row0 = s * batch;
-        m->steps++;
-        const float hp[3] = {lr, 1.0f - std::pow(0.9f, (float)m->steps), 1.0f - std::pow(0.999f, (float)m->steps)};
-        // pageable copies are staged by the driver before the call returns, so the host values may change
-        MCU(cudaMemcpyAsync(m->d_row0, &row0, sizeof row0, cudaMemcpyHostToDevice, st));
-        MCU(cudaMemcpyAsync(m->d_lr, hp, sizeof hp, cudaMemcpyHostToDevice, st));
-        MCU(cudaGraphLaunch(m->step_exec, st));
+    if (steps > m->hp_cap) {  // the captured step holds the old address
+        if (m->step_exec) cudaGraphExecDestroy(m->step_exec);
+        m->step_exec = nullptr;
+        cudaFree(m->d_hp);
+        m->d_hp = nullptr;
+        m->hp_cap = 0;
+        const long long cap = std::max(2 * steps, 256LL);
+        MCU(cudaMalloc((void**)&m->d_hp, (size_t)cap * sizeof(float4)));
+        m->hp_cap = cap;
     }
+    int rc = build_step_graph(m, batch);
+    if (rc != CLR_OK) return rc;
+    std::vector<float4> hp(steps);
+    for (long long s = 0; s < steps; ++s) {
+        m->steps++;
+        hp[s] = make_float4(lr, 1.0f - std::pow(0.9f, (float)m->steps), 1.0f - std::pow(0.999f, (float)m->steps), 0.0f);
+    }
+    const StepArgs args = {d_x, d_t, m->d_w, d_index, 0};
+    // pageable copies are staged by the driver before the calls return
+    MCU(cudaMemcpyAsync(m->d_step, &args, sizeof args, cudaMemcpyHostToDevice, st));
+    MCU(cudaMemcpyAsync(m->d_hp, hp.data(), (size_t)steps * sizeof(float4), cudaMemcpyHostToDevice, st));
+    MCU(cudaMemsetAsync(m->loss, 0, sizeof(float), st));
+    MCU(cudaEventRecord(m->ev0, st));
+    for (long long s = 0; s < steps; ++s) MCU(cudaGraphLaunch(m->step_exec, st));
     MCU(cudaEventRecord(m->ev1, st));
     float ls = 0.0f;
     MCU(cudaMemcpyAsync(&ls, m->loss, sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -1083,10 +1165,11 @@ extern "C" int clr_bf16_gemm_n256(const void* d_a, int64_t lda, const void* d_b,
     if (set_gemm_attributes() != cudaSuccess) return CLR_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) return CLR_ERR_CUDA;
-    GemmArgs g{};
+    GemmBatch b{};
+    GemmArgs& g = b.g[0];
     g.A = static_cast<const bf16*>(d_a); g.lda = lda; g.B = static_cast<const bf16*>(d_b); g.ldb = ldb;
     g.M = (int)M; g.K = (int)K; g.k_split = (int)K; g.out_f32 = d_c; g.ldo = ldc; g.err = err;
-    if (launch_gemm<EPI_STORE_F32>(g, 1, st) != cudaSuccess) return CLR_ERR_CUDA;
+    if (launch_gemm<EPI_STORE_F32>(b, 1, 1, st) != cudaSuccess) return CLR_ERR_CUDA;
     int herr = 0;
     if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return CLR_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return CLR_ERR_CUDA;
