@@ -373,15 +373,19 @@ __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict_
 // sums over odd and over even orders of a pi_n, b tau_n, a tau_n and b pi_n give S1 and S2 at mu and at
 // -mu: 8 FMAs per (bin, order) for both angles, against about 44 FP64 operations of the reference's order
 // of operations for the two. Tables differ from the reference-order ones by rounding only (tested).
-constexpr int kPdfFastGroup = 4;    // bins per block (one Legendre recurrence per angle serves them all)
+// kPdfFastGroup bins share a Legendre recurrence (8 operations per bin and order, 6 per order): 4 where there are
+// many bins and the FP64 pipe is the bound (96 % busy), 1 in one-warp blocks, the last bins first, where the largest
+// sizes' warps are (a warp issues one FP64 instruction per 64 cycles; see phase_pdf_kernel).
 constexpr int kPdfFastChunk = 128;  // orders staged per block
-__global__ void __launch_bounds__(128) phase_pdf_fast_kernel(const double* __restrict__ theta, int nt,
+template <int kPdfFastGroup, int kThreads>
+__global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* __restrict__ theta, int nt,
                                                              int n_particles, int order_cap,
                                                              const int* __restrict__ nstop,
                                                              const double* __restrict__ ab, double* __restrict__ pdf) {
     __shared__ double4 AB[kPdfFastGroup][kPdfFastChunk];
     __shared__ double2 RC[kPdfFastChunk];  // (2n+1)/n, (n+1)/n of the staged orders
-    const int g0 = blockIdx.y * kPdfFastGroup;
+    __shared__ double2 NF[kPdfFastChunk];  // n, -(n+1)
+    const int g0 = (int)(gridDim.y - 1 - blockIdx.y) * kPdfFastGroup;
     const int npair = (nt + 1) / 2;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = j < npair;
@@ -417,6 +421,7 @@ __global__ void __launch_bounds__(128) phase_pdf_fast_kernel(const double* __res
         for (int kk = threadIdx.x; kk < kPdfFastChunk; kk += blockDim.x) {
             const double nf = (double)(k0 + kk + 1);
             RC[kk] = make_double2((2.0 * nf + 1.0) / nf, (nf + 1.0) / nf);
+            NF[kk] = make_double2(nf, -(nf + 1.0));
         }
         __syncthreads();
         const int kend = min(kPdfFastChunk, kmax - k0);
@@ -426,8 +431,8 @@ __global__ void __launch_bounds__(128) phase_pdf_fast_kernel(const double* __res
         for (int kk = 0; kk < kend; kk += 2) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const double nf = (double)(k0 + kk + h + 1);
-                const double tau = fma(nf * mu, pi_n, -(nf + 1.0) * pi_nm1);
+                const double2 nf = NF[kk + h];
+                const double tau = fma(nf.x * mu, pi_n, nf.y * pi_nm1);
 #pragma unroll
                 for (int g = 0; g < kPdfFastGroup; ++g) {
                     const double4 q = AB[g][kk + h];
@@ -1460,8 +1465,13 @@ cudaError_t enqueue_mie_tables(const double* d, const double* nr, const double* 
     if (hybrid) {
         theta_grid_kernel<<<(nt + 127) / 128, 128, 0, st>>>(b.theta, b.theta_f, nt);
         if (fast_pdf) {
-            dim3 grid(((nt + 1) / 2 + 127) / 128, (n + kPdfFastGroup - 1) / kPdfFastGroup);
-            phase_pdf_fast_kernel<<<grid, 128, 0, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, b.pdf);
+            const int pairs = (nt + 1) / 2;
+            if (n < kPdfManyBins)
+                phase_pdf_fast_kernel<1, 32><<<dim3((pairs + 31) / 32, n), 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop,
+                                                                                      b.ab, b.pdf);
+            else
+                phase_pdf_fast_kernel<4, 128><<<dim3((pairs + 127) / 128, (n + 3) / 4), 128, 0, st>>>(
+                    b.theta, nt, n, order_cap, b.nstop, b.ab, b.pdf);
         } else {
             if (n < kPdfManyBins)
                 phase_pdf_kernel<1><<<dim3((nt + 31) / 32, n), 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, b.pdf);
