@@ -429,23 +429,30 @@ struct XorMode {
         m->s = D.det_seed + gid * 3266489917u + 668265263u;
     }
 };
-struct PhiloxMode {
-    using Stream = PhiloxStream;
+template <class P>
+struct PhiloxModeOf {
+    using Stream = P;
     struct Lane {
-        PhiloxStream p;
-        __device__ __forceinline__ PhiloxStream* transport() { return &p; }
-        __device__ __forceinline__ PhiloxStream* optics() { return &p; }
-        __device__ __forceinline__ PhiloxStream* source() { return &p; }
+        P p;
+        __device__ __forceinline__ P* transport() { return &p; }
+        __device__ __forceinline__ P* optics() { return &p; }
+        __device__ __forceinline__ P* source() { return &p; }
     };
     __device__ __forceinline__ static void seed(const DevScene& D, uint32_t gid, Lane& L) {
         L.p.init(D.philox_key, gid, D.scenario_id, 0u);
     }
-    __device__ __forceinline__ static void detector_streams(const DevScene& D, uint32_t gid, PhiloxStream* n,
-                                                            PhiloxStream* m) {
+    __device__ __forceinline__ static void detector_streams(const DevScene& D, uint32_t gid, P* n, P* m) {
         n->init(D.philox_key, gid, D.scenario_id, 1u);
         m->init(D.philox_key, gid, D.scenario_id, 2u);
     }
 };
+using PhiloxMode = PhiloxModeOf<PhiloxStream>;
+using PhiloxCallMode = PhiloxModeOf<PhiloxCallStream>;
+static_assert(sizeof(PhiloxMode::Lane) == sizeof(PhiloxCallMode::Lane), "one layout of the stream's state");
+// The mode of the stages without closures: a serial closure's results depend in their last bits on how the compiler
+// contracts the code around its draws, so the closures keep the inlined stream.
+template <class Mode> struct LeanMode { using type = Mode; };
+template <> struct LeanMode<PhiloxMode> { using type = PhiloxCallMode; };
 
 __device__ __forceinline__ void flush_warp_tally(WarpTally* t, DevTally* dst, int lane) {
     unsigned long long* su = &t->hw[0][0];
