@@ -34,6 +34,8 @@ struct clr_ctx {
     unsigned long long* d_work = nullptr;
     int num_sms = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaStream_t side = nullptr;  // work of a scene build beside the main stream's
+    cudaEvent_t side_ev[2] = {nullptr, nullptr};
     float last_kernel_ms = 0.0f;
     // wavefront engine pool (allocated on first use)
     unsigned wave_cap = 0;
@@ -129,6 +131,8 @@ int clr_create(clr_ctx** out, int device) {
     }
     CU(cudaEventCreate(&ctx->ev0));
     CU(cudaEventCreate(&ctx->ev1));
+    CU(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : ctx->side_ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     *out = ctx;
     return CLR_OK;
 }
@@ -136,6 +140,7 @@ int clr_create(clr_ctx** out, int device) {
 int clr_destroy(clr_ctx* ctx) {
     if (!ctx) return CLR_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
+    if (ctx->side) cudaStreamSynchronize(ctx->side);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     free_particles(ctx);
     cudaFree(ctx->d_scene);
@@ -161,6 +166,9 @@ int clr_destroy(clr_ctx* ctx) {
         if (e) cudaEventDestroy(e);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+    for (cudaEvent_t e : ctx->side_ev)
+        if (e) cudaEventDestroy(e);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return CLR_OK;
@@ -318,7 +326,11 @@ int clr_build_particles(clr_ctx* ctx, const clr_particle_spec* ps, const clr_sed
     CU(dalloc(ctx, (void**)&pb.nstop, n * sizeof(int)));
     CU(dalloc(ctx, (void**)&pb.moment_mode, n));
     CU(dalloc(ctx, (void**)&pb.err, sizeof(int)));
-    CU(D(&pb.ab, (size_t)n * CLR_MIE_MAX_ORDER * 4));
+    const int cap = particle_order_cap(*ps);
+    CU(D(&pb.ab, (size_t)n * cap * 4));
+    if (hybrid_model(sp))
+        if (const size_t bytes = legendre_table_bytes(nt, cap, ps->table_arithmetic == CLR_TABLES_FAST))
+            CU(dalloc(ctx, (void**)&pb.legendre, bytes));
     CU(D(&pb.theta, nt));
     CU(F(&pb.theta_f, nt));
     CU(D(&pb.pdf, (size_t)n * nt));
@@ -369,7 +381,7 @@ int clr_build_particles(clr_ctx* ctx, const clr_particle_spec* ps, const clr_sed
         const double one[4] = {1.0, 1.0, 1.0, 1.0};
         CU(cudaMemcpyAsync(pb.sed_grid, one, sizeof(double), cudaMemcpyHostToDevice, st));
     }
-    CU(enqueue_particle_precompute(pb, sp, *ps, *ss, nullptr, st));  // ss: FP64 geometry filled
+    CU(enqueue_particle_precompute(pb, sp, *ps, *ss, {ctx->side, ctx->side_ev[0], ctx->side_ev[1]}, st));  // ss: FP64 geometry filled
     int herr = 0;
     CU(cudaMemcpyAsync(&herr, pb.err, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (pb.node_tables)
@@ -913,7 +925,9 @@ static int sweep_build(clr_ctx* ctx, int ns, const clr_scene_params* sps, const 
     // Mie tables: chunks of at most kSweepChunkBins bins within each run of scenarios sharing the key
     struct Chunk { int s0; long long b0, b1; int cap; };
     std::vector<Chunk> chunks;
-    size_t scratch = 0;
+    size_t scratch = 0, table_bytes = 0;
+    const bool fast = pss[0].table_arithmetic == CLR_TABLES_FAST;
+    std::vector<int> group_cap(L.group_first.size(), 1);  // largest order bound of a group: its table serves its chunks
     for (size_t g = 0; g + 1 < L.group_first.size(); ++g) {
         const int s0 = L.group_first[g], s1 = L.group_first[g + 1];
         const clr_particle_spec& ps = pss[s0];
@@ -922,11 +936,15 @@ static int sweep_build(clr_ctx* ctx, int ns, const clr_scene_params* sps, const 
             const int cap = mie_order_bound(hd.data() + b0, hn.data() + b0, hk.data() + b0, (int)(b1 - b0),
                                             ps.n_medium, ps.wavelength_m);
             chunks.push_back({s0, b0, b1, cap});
+            group_cap[g] = std::max(group_cap[g], cap);
             const size_t ab = (size_t)(b1 - b0) * cap * 4 * sizeof(double);
             const size_t pdf = hybrid_model(sps[s0]) ? (size_t)(b1 - b0) * pbs[s0].nt * sizeof(double) : 0;
             scratch = std::max(scratch, ((ab + 255) & ~(size_t)255) + pdf);
         }
+        if (hybrid_model(sps[s0]))
+            table_bytes = std::max(table_bytes, (legendre_table_bytes(pbs[s0].nt, group_cap[g], fast) + 255) & ~(size_t)255);
     }
+    scratch += table_bytes;
     if (scratch > ctx->sw_scratch_bytes) {
         CU(cudaStreamSynchronize(st));
         cudaFree(ctx->sw_scratch);
@@ -935,13 +953,24 @@ static int sweep_build(clr_ctx* ctx, int ns, const clr_scene_params* sps, const 
         CU(cudaMalloc(&ctx->sw_scratch, scratch));
         ctx->sw_scratch_bytes = scratch;
     }
+    double2* const table = static_cast<double2*>(ctx->sw_scratch);
+    char* const chunk_scratch = static_cast<char*>(ctx->sw_scratch) + table_bytes;
+    size_t group = 0;
+    int table_of = -1;  // first scenario of the group whose table is there
     for (const Chunk& c : chunks) {
+        while (c.s0 >= L.group_first[group + 1]) ++group;
         const ParticleBuffers& G = pbs[c.s0];
+        const bool tabled = hybrid_model(sps[c.s0]) && legendre_table_bytes(G.nt, group_cap[group], fast) > 0;
+        if (tabled && table_of != c.s0) {
+            CU(enqueue_legendre_table(G.theta, G.theta_f, G.nt, group_cap[group], fast, table, st));
+            table_of = c.s0;
+        }
         const long long nb = c.b1 - c.b0;
         const long long tab = L.tab_off[c.s0] + (c.b0 - L.bin_off[c.s0]) * G.nt;
         MiePhaseBuffers b;
-        b.ab = static_cast<double*>(ctx->sw_scratch);
-        b.pdf = reinterpret_cast<double*>(static_cast<char*>(ctx->sw_scratch) +
+        if (tabled) b.table = table;
+        b.ab = reinterpret_cast<double*>(chunk_scratch);
+        b.pdf = reinterpret_cast<double*>(chunk_scratch +
                                           (((size_t)nb * c.cap * 4 * sizeof(double) + 255) & ~(size_t)255));
         b.nstop = P0.nstop + c.b0; b.x = P0.x + c.b0; b.qext = P0.qext + c.b0; b.qsca = P0.qsca + c.b0;
         b.qabs = P0.qabs + c.b0; b.qback = P0.qback + c.b0; b.g = P0.g + c.b0; b.albedo = P0.albedo + c.b0;

@@ -112,7 +112,8 @@ struct ParticleBuffers {
     int* nstop = nullptr;
     double *x = nullptr, *qext = nullptr, *qsca = nullptr, *qabs = nullptr, *qback = nullptr, *g = nullptr,
            *albedo = nullptr;
-    double* ab = nullptr;  // Mie a_n, b_n scratch: [n][CLR_MIE_MAX_ORDER][4] (a.re, a.im, b.re, b.im)
+    double* ab = nullptr;  // Mie a_n, b_n scratch: [n][order bound][4] (a.re, a.im, b.re, b.im)
+    double2* legendre = nullptr;  // table of the angular functions (legendre_table_bytes)
     double *theta = nullptr, *pdf = nullptr, *phase_cdf = nullptr;
     float *theta_f = nullptr, *phase_cdf_f = nullptr;
     int* phase_guide = nullptr;  // [n][kPhaseGuide + 1]
@@ -156,6 +157,10 @@ struct MiePhaseBuffers {
     double* cdf;      // [n][nt]
     float* cdf_f;     // [n][nt]
     int* guide = nullptr;  // [n][kPhaseGuide + 1] search guide of cdf_f, or null (not built)
+    // pi_n, tau_n of every angle and order (enqueue_legendre_table, which then also made the theta grid), ready when
+    // table_ready (if any) is; without it the pdf kernels run the recurrence themselves
+    const double2* table = nullptr;
+    cudaEvent_t table_ready = nullptr;
     int* err;         // error word, cleared by the call
 };
 cudaError_t enqueue_mie_phase(const double* d, const double* nr, const double* k, int n, double n_medium,
@@ -166,8 +171,13 @@ cudaError_t enqueue_mie_phase(const double* d, const double* nr, const double* k
 cudaError_t enqueue_mie_tables(const double* d, const double* nr, const double* k, int n, double n_medium,
                                double wavelength, int nt, bool hybrid, int order_cap, const MiePhaseBuffers& b,
                                cudaStream_t stream, bool fast_pdf = false);
+// The theta grid and the table of the angular functions for bins of this order bound (0 bytes: too large, no table).
+size_t legendre_table_bytes(int nt, int order_cap, bool fast);
+cudaError_t enqueue_legendre_table(double* theta, float* theta_f, int nt, int order_cap, bool fast, double2* table,
+                                   cudaStream_t stream);
 // Orders the Mie kernel needs for these bins (host arithmetic, with slack), at most CLR_MIE_MAX_ORDER.
 int mie_order_bound(const double* d, const double* nr, const double* k, int n, double n_medium, double wavelength);
+int particle_order_cap(const clr_particle_spec& ps);
 // Precompute error code of a Mie launch whose order bound was too small (not a reference code).
 #define CLR_ERR_CODE_ORDER_CAP 90
 
@@ -182,9 +192,13 @@ struct NoallocScratch {
 cudaError_t noalloc_scratch(int device, NoallocScratch* out);
 
 // Enqueue the whole precompute on `stream`. Host inputs are copied in; error codes land in pb.err.
-// `ab_scratch` may supply the Mie a_n/b_n scratch (n*CLR_MIE_MAX_ORDER*4 doubles); when null, pb.ab is used.
+// `side`: a stream of the caller for work that runs beside it, and two events.
+struct SideStream {
+    cudaStream_t stream;
+    cudaEvent_t start, done;
+};
 cudaError_t enqueue_particle_precompute(ParticleBuffers& pb, const clr_scene_params& sp, const clr_particle_spec& ps,
-                                        const clr_sediment_spec& ss, double* ab_scratch, cudaStream_t stream);
+                                        const clr_sediment_spec& ss, const SideStream& side, cudaStream_t stream);
 // The meridional advection-diffusion field of sediment model 3 (one cooperative launch, a CTA per bin)
 // into pb.sed_grid and pb.grid_max; pb.merid_* must be allocated (meridional_coef_doubles coefficients).
 size_t meridional_coef_doubles(int n, int nr, int nz);

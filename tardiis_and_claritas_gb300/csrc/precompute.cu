@@ -291,27 +291,67 @@ __global__ void theta_grid_kernel(double* theta, float* theta_f, int nt) {
     theta_f[j] = (float)v;
 }
 
+// pi_n, tau_n of every angle and order (:3561-3581), the same for every bin: table[n - 1][angle], `pitch` angles apart
+// (a multiple of 32). One warp per 32 angles: the recurrence is a chain of 8 (kFast: 6, with fused multiply-adds) FP64
+// operations per order, which every warp of the pdf kernels would repeat for its own bins (8 of 28 operations with a
+// bin per warp, 8 of 88 with four); from the table (L2-resident) they only load. The quotients of an order are
+// identical to evaluating them inline.
+constexpr int kLegStage = 64;
+template <bool kFast>
+__global__ void __launch_bounds__(32) legendre_table_kernel(const double* __restrict__ theta, int angles, int rows,
+                                                            int pitch, double2* __restrict__ table) {
+    __shared__ double QN[4][kLegStage];  // n, n+1, (2n+1)/n, (n+1)/n
+    const int lane = threadIdx.x, j = blockIdx.x * 32 + lane;
+    const double mu = j < angles ? cos(theta[j]) : 0.0;
+    double pi_nm1 = 0.0, pi_n = 1.0;
+    for (int k0 = 0; k0 < rows; k0 += kLegStage) {
+        __syncwarp();
+#pragma unroll
+        for (int kk = lane; kk < kLegStage; kk += 32) {
+            const double nf = (double)(k0 + kk + 1);
+            QN[0][kk] = nf; QN[1][kk] = nf + 1.0;
+            QN[2][kk] = (2.0 * nf + 1.0) / nf;
+            QN[3][kk] = (nf + 1.0) / nf;
+        }
+        __syncwarp();
+        const int kend = min(kLegStage, rows - k0);
+        for (int kk = 0; kk < kend; ++kk) {
+            double tau, pi_np1;
+            if constexpr (kFast) {
+                tau = fma(QN[0][kk] * mu, pi_n, -QN[1][kk] * pi_nm1);
+                pi_np1 = fma(QN[2][kk] * mu, pi_n, -QN[3][kk] * pi_nm1);
+            } else {
+                tau = QN[0][kk] * mu * pi_n - QN[1][kk] * pi_nm1;
+                pi_np1 = QN[2][kk] * mu * pi_n - QN[3][kk] * pi_nm1;
+            }
+            table[(size_t)(k0 + kk) * pitch + j] = make_double2(pi_n, tau);
+            pi_nm1 = pi_n; pi_n = pi_np1;
+        }
+    }
+}
+
 // S1/S2 -> 0.5(|S1|^2+|S2|^2) sin(theta) for kPdfGroup bins at one angle per lane (:3561-3581). Bound by the FP64
-// pipe (20 operations per bin and order, 8 per order for the angular recurrence that the bins share; no contraction).
+// pipe (20 operations per bin and order; without the table of pi_n, tau_n 8 more per order; no contraction).
 // A warp issues one FP64 instruction per 64 cycles, so few bins make the largest sizes' warps the longest: with four
 // bins to a warp in blocks of 128 angles, the last blocks of 63 bins ran 4.4 ms where the pipe's work is 1.2 ms.
 // One warp per block, the last bins (usually the largest, with the most orders) first, and kPdfGroup = 1 below
-// kPdfManyBins bins (28 operations per bin and order, an even load), 4 above (22, and enough blocks to even out).
+// kPdfManyBins bins (an even load), 4 above (fewer loads, and enough blocks to even out).
 // Coefficients and the quotients of an order (identical to evaluating them inline) are staged kPdfStage orders at
 // a time.
 constexpr int kPdfManyBins = 608;
 constexpr int kPdfPad = 14 * 1024;  // unused shared memory per block of one bin: 12 blocks per SM, the rest wait, so
                                     // that a partition whose warps end early takes the next (2.78 ms with all resident)
 constexpr int kPdfStage = 64;
-template <int kPdfGroup>
+template <int kPdfGroup, bool kTable>
 __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict__ theta, int nt, int n_particles,
                                                        int order_cap, const int* __restrict__ nstop,
-                                                       const double* __restrict__ ab, double* __restrict__ pdf) {
+                                                       const double* __restrict__ ab, const double2* __restrict__ table,
+                                                       int pitch, double* __restrict__ pdf) {
     __shared__ double4 AB[kPdfGroup][kPdfStage];
     __shared__ double QN[5][kPdfStage];  // n, n+1, (2n+1)/(n(n+1)), (2n+1)/n, (n+1)/n
     const int lane = threadIdx.x, j = blockIdx.x * 32 + lane;
     const int g0 = (int)(gridDim.y - 1 - blockIdx.y) * kPdfGroup;
-    const double th = j < nt ? theta[j] : 0.0, mu = cos(th);
+    const double th = j < nt ? theta[j] : 0.0, mu = kTable ? 0.0 : cos(th);
     double s1r[kPdfGroup], s1i[kPdfGroup], s2r[kPdfGroup], s2i[kPdfGroup];
     int ns[kPdfGroup];
     int kmax = 0;
@@ -323,16 +363,20 @@ __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict_
     }
     const double4* abp = reinterpret_cast<const double4*>(ab);
     double pi_nm1 = 0.0, pi_n = 1.0;
+    double2 pt = make_double2(0.0, 0.0);
+    if (kTable && kmax > 0) pt = table[j];
     for (int k0 = 0; k0 < kmax; k0 += kPdfStage) {
         __syncwarp();
 #pragma unroll
         for (int h = 0; h < kPdfStage; h += 32) {
             const int kk = h + lane, k = k0 + kk;
             const double nf = (double)(k + 1);
-            QN[0][kk] = nf; QN[1][kk] = nf + 1.0;
             QN[2][kk] = (2.0 * nf + 1.0) / (nf * (nf + 1.0));
-            QN[3][kk] = (2.0 * nf + 1.0) / nf;
-            QN[4][kk] = (nf + 1.0) / nf;
+            if constexpr (!kTable) {
+                QN[0][kk] = nf; QN[1][kk] = nf + 1.0;
+                QN[3][kk] = (2.0 * nf + 1.0) / nf;
+                QN[4][kk] = (nf + 1.0) / nf;
+            }
 #pragma unroll
             for (int g = 0; g < kPdfGroup; ++g)
                 if (k < ns[g]) AB[g][kk] = abp[(size_t)(g0 + g) * order_cap + k];
@@ -340,7 +384,14 @@ __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict_
         __syncwarp();
         const int kend = min(kPdfStage, kmax - k0);
         for (int kk = 0; kk < kend; ++kk) {
-            const double tau = QN[0][kk] * mu * pi_n - QN[1][kk] * pi_nm1, c = QN[2][kk];
+            double tau;
+            if constexpr (kTable) {
+                pi_n = pt.x; tau = pt.y;
+                if (k0 + kk + 1 < kmax) pt = table[(size_t)(k0 + kk + 1) * pitch + j];
+            } else {
+                tau = QN[0][kk] * mu * pi_n - QN[1][kk] * pi_nm1;
+            }
+            const double c = QN[2][kk];
 #pragma unroll
             for (int g = 0; g < kPdfGroup; ++g) {
                 if (k0 + kk < ns[g]) {
@@ -352,8 +403,10 @@ __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict_
                     s2i[g] += c * (ai * tau + bi * pi_n);
                 }
             }
-            const double pi_np1 = QN[3][kk] * mu * pi_n - QN[4][kk] * pi_nm1;
-            pi_nm1 = pi_n; pi_n = pi_np1;
+            if constexpr (!kTable) {
+                const double pi_np1 = QN[3][kk] * mu * pi_n - QN[4][kk] * pi_nm1;
+                pi_nm1 = pi_n; pi_n = pi_np1;
+            }
         }
     }
     if (j >= nt) return;
@@ -373,18 +426,20 @@ __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict_
 // sums over odd and over even orders of a pi_n, b tau_n, a tau_n and b pi_n give S1 and S2 at mu and at
 // -mu: 8 FMAs per (bin, order) for both angles, against about 44 FP64 operations of the reference's order
 // of operations for the two. Tables differ from the reference-order ones by rounding only (tested).
-// kPdfFastGroup bins share a Legendre recurrence (8 operations per bin and order, 6 per order): 4 where there are
-// many bins and the FP64 pipe is the bound (96 % busy), 1 in one-warp blocks, the last bins first, where the largest
-// sizes' warps are (a warp issues one FP64 instruction per 64 cycles; see phase_pdf_kernel).
+// pi_n and tau_n come from the table. kPdfFastGroup bins share their loads: 4 where there are many bins and the FP64
+// pipe is the bound, 1 in one-warp blocks, the last bins first, where the largest sizes' warps are (a warp issues one
+// FP64 instruction per 64 cycles; see phase_pdf_kernel).
 constexpr int kPdfFastChunk = 128;  // orders staged per block
-template <int kPdfFastGroup, int kThreads>
+template <int kPdfFastGroup, int kThreads, bool kTable>
 __global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* __restrict__ theta, int nt,
                                                              int n_particles, int order_cap,
                                                              const int* __restrict__ nstop,
-                                                             const double* __restrict__ ab, double* __restrict__ pdf) {
+                                                             const double* __restrict__ ab,
+                                                             const double2* __restrict__ table, int pitch,
+                                                             double* __restrict__ pdf) {
     __shared__ double4 AB[kPdfFastGroup][kPdfFastChunk];
-    __shared__ double2 RC[kPdfFastChunk];  // (2n+1)/n, (n+1)/n of the staged orders
-    __shared__ double2 NF[kPdfFastChunk];  // n, -(n+1)
+    __shared__ double2 RC[kTable ? 1 : kPdfFastChunk];  // without the table: (2n+1)/n, (n+1)/n of the staged orders
+    __shared__ double2 NF[kTable ? 1 : kPdfFastChunk];  // n, -(n+1)
     const int g0 = (int)(gridDim.y - 1 - blockIdx.y) * kPdfFastGroup;
     const int npair = (nt + 1) / 2;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -396,7 +451,6 @@ __global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* 
         ns[g] = (g0 + g < n_particles) ? nstop[g0 + g] : 0;
         kmax = ns[g] > kmax ? ns[g] : kmax;
     }
-    const double mu = active ? cos(theta[j]) : 0.0;
     // per bin: odd-order sums P = a pi, Q = b tau, R = a tau, T = b pi (re, im), then the even-order ones
     double acc[kPdfFastGroup][16];
 #pragma unroll
@@ -404,6 +458,12 @@ __global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* 
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[g][i] = 0.0;
     const double4* ab4 = reinterpret_cast<const double4*>(ab);
+    // threads past the last pair of angles read the row's padding (or its last angle) and store nothing
+    const double2* const col = kTable ? table + min(j, pitch - 1) : nullptr;
+    double2 next[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    if (kTable && kmax > 0) next[0] = col[0];
+    if (kTable && kmax > 1) next[1] = col[pitch];
+    const double mu = !kTable && active ? cos(theta[j]) : 0.0;
     double pi_nm1 = 0.0, pi_n = 1.0;
     for (int k0 = 0; k0 < kmax; k0 += kPdfFastChunk) {
         __syncthreads();
@@ -418,11 +478,12 @@ __global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* 
             }
             AB[g][kk] = v;
         }
-        for (int kk = threadIdx.x; kk < kPdfFastChunk; kk += blockDim.x) {
-            const double nf = (double)(k0 + kk + 1);
-            RC[kk] = make_double2((2.0 * nf + 1.0) / nf, (nf + 1.0) / nf);
-            NF[kk] = make_double2(nf, -(nf + 1.0));
-        }
+        if constexpr (!kTable)
+            for (int kk = threadIdx.x; kk < kPdfFastChunk; kk += blockDim.x) {
+                const double nf = (double)(k0 + kk + 1);
+                RC[kk] = make_double2((2.0 * nf + 1.0) / nf, (nf + 1.0) / nf);
+                NF[kk] = make_double2(nf, -(nf + 1.0));
+            }
         __syncthreads();
         const int kend = min(kPdfFastChunk, kmax - k0);
         // k0 is even, so order n = k0 + kk + 1 is odd for even kk: odd-order sums go to acc[g][0..7], even-order
@@ -431,8 +492,13 @@ __global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* 
         for (int kk = 0; kk < kend; kk += 2) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const double2 nf = NF[kk + h];
-                const double tau = fma(nf.x * mu, pi_n, nf.y * pi_nm1);
+                double tau;
+                if constexpr (kTable) {
+                    pi_n = next[h].x; tau = next[h].y;
+                    if (k0 + kk + h + 2 < kmax) next[h] = col[(size_t)(k0 + kk + h + 2) * pitch];
+                } else {
+                    tau = fma(NF[kk + h].x * mu, pi_n, NF[kk + h].y * pi_nm1);
+                }
 #pragma unroll
                 for (int g = 0; g < kPdfFastGroup; ++g) {
                     const double4 q = AB[g][kk + h];
@@ -442,9 +508,10 @@ __global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* 
                     A[4] = fma(q.x, tau, A[4]);  A[5] = fma(q.y, tau, A[5]);   // R
                     A[6] = fma(q.z, pi_n, A[6]); A[7] = fma(q.w, pi_n, A[7]);  // T
                 }
-                const double2 rc = RC[kk + h];
-                const double pi_np1 = fma(rc.x * mu, pi_n, -rc.y * pi_nm1);
-                pi_nm1 = pi_n; pi_n = pi_np1;
+                if constexpr (!kTable) {
+                    const double pi_np1 = fma(RC[kk + h].x * mu, pi_n, -RC[kk + h].y * pi_nm1);
+                    pi_nm1 = pi_n; pi_n = pi_np1;
+                }
             }
         }
     }
@@ -1443,12 +1510,38 @@ int mie_order_bound(const double* d, const double* nr, const double* k, int n, d
     return std::min(cap, (int)CLR_MIE_MAX_ORDER);
 }
 
+int particle_order_cap(const clr_particle_spec& ps) {
+    return mie_order_bound(ps.diameter_m, ps.n_real, ps.k_imag, ps.n_bins, ps.n_medium, ps.wavelength_m);
+}
+
 static cudaError_t set_table_attributes() {
     cudaError_t e = cudaFuncSetAttribute(mie_coefficients_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kMieSmem);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(phase_cdf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(kCdfSmemAngles * sizeof(double)));
+}
+
+// Angles per row of a Legendre table (the fast tables mirror angles: half of them), and its orders for bins of a
+// launch with this order bound (the bound holds the 128 extra orders of the downward recurrence).
+static int legendre_pitch(int nt, bool fast) { return ((fast ? (nt + 1) / 2 : nt) + 31) & ~31; }
+static int legendre_rows(int order_cap) {
+    return order_cap >= CLR_MIE_MAX_ORDER ? CLR_MIE_MAX_ORDER : std::max(order_cap - 128, 1);
+}
+// No table above kLegendreMaxBytes (1801 angles and 1500 orders take 43 MB, which L2 holds; the table grows with the
+// angles times the orders, which no other array does).
+constexpr size_t kLegendreMaxBytes = (size_t)256 << 20;
+size_t legendre_table_bytes(int nt, int order_cap, bool fast) {
+    const size_t bytes = (size_t)legendre_rows(order_cap) * legendre_pitch(nt, fast) * sizeof(double2);
+    return bytes <= kLegendreMaxBytes ? bytes : 0;
+}
+cudaError_t enqueue_legendre_table(double* theta, float* theta_f, int nt, int order_cap, bool fast, double2* table,
+                                   cudaStream_t st) {
+    const int pitch = legendre_pitch(nt, fast), rows = legendre_rows(order_cap);
+    theta_grid_kernel<<<(nt + 127) / 128, 128, 0, st>>>(theta, theta_f, nt);
+    if (fast) legendre_table_kernel<true><<<pitch / 32, 32, 0, st>>>(theta, (nt + 1) / 2, rows, pitch, table);
+    else legendre_table_kernel<false><<<pitch / 32, 32, 0, st>>>(theta, nt, rows, pitch, table);
+    return cudaGetLastError();
 }
 
 // Mie coefficients and efficiencies of n bins, then (hybrid event models) the theta grid and the phase
@@ -1463,21 +1556,24 @@ cudaError_t enqueue_mie_tables(const double* d, const double* nr, const double* 
         d, nr, k, n_medium, wavelength, n, order_cap, b.ab, b.nstop, b.x, b.qext, b.qsca, b.qabs, b.qback, b.g,
         b.albedo, b.err);
     if (hybrid) {
-        theta_grid_kernel<<<(nt + 127) / 128, 128, 0, st>>>(b.theta, b.theta_f, nt);
+        if (!b.table) theta_grid_kernel<<<(nt + 127) / 128, 128, 0, st>>>(b.theta, b.theta_f, nt);
+        else if (b.table_ready && (e = cudaStreamWaitEvent(st, b.table_ready, 0)) != cudaSuccess) return e;
+        const dim3 one((nt + 31) / 32, n), four((nt + 31) / 32, (n + 3) / 4);
+        const int pairs = (nt + 1) / 2, pitch = legendre_pitch(nt, fast_pdf);
         if (fast_pdf) {
-            const int pairs = (nt + 1) / 2;
-            if (n < kPdfManyBins)
-                phase_pdf_fast_kernel<1, 32><<<dim3((pairs + 31) / 32, n), 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop,
-                                                                                      b.ab, b.pdf);
-            else
-                phase_pdf_fast_kernel<4, 128><<<dim3((pairs + 127) / 128, (n + 3) / 4), 128, 0, st>>>(
-                    b.theta, nt, n, order_cap, b.nstop, b.ab, b.pdf);
+            auto fast = [&](auto kernel, int group, int threads, size_t pad) {
+                kernel<<<dim3((pairs + threads - 1) / threads, (n + group - 1) / group), threads, pad, st>>>(
+                    b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
+            };
+            if (!b.table) fast(phase_pdf_fast_kernel<1, 32, false>, 1, 32, kPdfPad);
+            else if (n < kPdfManyBins) fast(phase_pdf_fast_kernel<1, 32, true>, 1, 32, kPdfPad);
+            else fast(phase_pdf_fast_kernel<4, 128, true>, 4, 128, 0);
+        } else if (!b.table) {
+            phase_pdf_kernel<1, false><<<one, 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, nullptr, 0, b.pdf);
+        } else if (n < kPdfManyBins) {
+            phase_pdf_kernel<1, true><<<one, 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
         } else {
-            if (n < kPdfManyBins)
-                phase_pdf_kernel<1><<<dim3((nt + 31) / 32, n), 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, b.pdf);
-            else
-                phase_pdf_kernel<4><<<dim3((nt + 31) / 32, (n + 3) / 4), 32, 0, st>>>(b.theta, nt, n, order_cap, b.nstop,
-                                                                                       b.ab, b.pdf);
+            phase_pdf_kernel<4, true><<<four, 32, 0, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
         }
         const size_t row = nt <= kCdfSmemAngles ? (size_t)nt * sizeof(double) : 0;
         phase_cdf_kernel<<<n, kCdfThreads, row, st>>>(b.theta, b.pdf, nt, n, b.cdf, b.cdf_f, b.err);
@@ -1608,19 +1704,27 @@ cudaError_t enqueue_scene_rates_batch(ParticleBuffers* const* pbs, const clr_sce
 }
 
 cudaError_t enqueue_particle_precompute(ParticleBuffers& pb, const clr_scene_params& sp, const clr_particle_spec& ps,
-                                        const clr_sediment_spec& ss, double* ab_scratch, cudaStream_t st) {
+                                        const clr_sediment_spec& ss, const SideStream& side, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(pb.err, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     MiePhaseBuffers b;
-    b.ab = ab_scratch ? ab_scratch : pb.ab;
+    b.ab = pb.ab;
     b.nstop = pb.nstop; b.x = pb.x; b.qext = pb.qext; b.qsca = pb.qsca; b.qabs = pb.qabs; b.qback = pb.qback;
     b.g = pb.g; b.albedo = pb.albedo; b.theta = pb.theta; b.theta_f = pb.theta_f; b.pdf = pb.pdf;
     b.cdf = pb.phase_cdf; b.cdf_f = pb.phase_cdf_f; b.guide = pb.phase_guide; b.err = pb.err;
     const int em = sp.event_model;
-    e = enqueue_mie_tables(pb.d, pb.nidx, pb.kidx, pb.n, ps.n_medium, ps.wavelength_m, pb.nt,
-                           em == 3 || em == 4 || em == 5,
-                           mie_order_bound(ps.diameter_m, ps.n_real, ps.k_imag, pb.n, ps.n_medium, ps.wavelength_m), b,
-                           st, ps.table_arithmetic == CLR_TABLES_FAST);
+    const bool hybrid = em == 3 || em == 4 || em == 5, fast = ps.table_arithmetic == CLR_TABLES_FAST;
+    const int cap = particle_order_cap(ps);
+    if (hybrid && pb.legendre) {  // the angular functions beside the Mie coefficients, which leave most SMs free
+        b.table = pb.legendre;
+        b.table_ready = side.done;
+        if ((e = cudaEventRecord(side.start, st)) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(side.stream, side.start, 0)) != cudaSuccess) return e;
+        if ((e = enqueue_legendre_table(pb.theta, pb.theta_f, pb.nt, cap, fast, pb.legendre, side.stream)) != cudaSuccess)
+            return e;
+        if ((e = cudaEventRecord(side.done, side.stream)) != cudaSuccess) return e;
+    }
+    e = enqueue_mie_tables(pb.d, pb.nidx, pb.kidx, pb.n, ps.n_medium, ps.wavelength_m, pb.nt, hybrid, cap, b, st, fast);
     if (e != cudaSuccess) return e;
     return enqueue_scene_rates(pb, sp, ps, ss, st);
 }
