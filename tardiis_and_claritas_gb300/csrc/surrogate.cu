@@ -584,39 +584,43 @@ __global__ void adam_kernel(float* params, float* grads, float* m1, float* m2, c
 }
 
 // ---------------- fused inference: every layer of a 128-row tile on one SM ----------------
-// A persistent CTA per SM walks 128-row tiles, with every product on the tensor cores: layer 1 as one
-// tcgen05.mma with K padded from 6 to 16, the three 256x256 layers as 16 MMAs each, and the 256 -> 3
-// output layer as 16 MMAs with N padded to 16. The small padded weight images (W1, W5) stay in shared
-// memory; each 256x256 weight image (128 KB) comes in by one cp.async.bulk copy that starts as soon as
-// the previous layer's MMAs have completed, so it overlaps that layer's epilogue. Each epilogue reads the
-// accumulator with tcgen05.ld, adds the bias, applies SiLU (one tanh.approx per element) and writes the
-// next layer's A image. Activations never leave the SM.
-constexpr int kInferThreads = 512;               // warp w reads TMEM lane quarter w % 4, columns 64 (w / 4) ..
-constexpr int kABytes = kM * kHid * 2;           // 64 KB: the tile's activations, K = 256
-constexpr int kWBytes = kHid * kHid * 2;         // 128 KB: one 256x256 weight image
+// A persistent CTA per SM walks 128-row tiles with every product on the tensor cores: layer 1 with K padded from 6
+// to 16, three 256x256 layers, the 256 -> 3 output layer with N padded to 16. What bounds it is the SiLU: one
+// multi-function operation per activation, 16 a clock and SM, 2048 cycles per layer and tile, against 1024 for the
+// layer's MMAs. So the MMAs run under the epilogues: a layer's 256 outputs are two halves of 128 columns; while
+// sixteen warps turn half 0 of layer l into activations, a warp of its own has the tensor cores make half 1, and
+// while they work on half 1, the first half of layer l + 1's K. Activations stay in tensor memory (two images of
+// 128 columns, the accumulator the other 256), from where tcgen05.mma takes its A operand, which leaves shared
+// memory to the weights: a ring of three half layers (64 KB each, one bulk copy), refilled as each half's MMAs end.
+// With the activations in shared memory, one weight buffer and each layer's MMAs, copy and epilogue one after the
+// other, 65536 queries took 52 us.
+constexpr int kInferWarps = 16;                  // epilogue warps: TMEM lane quarter w % 4, 32 columns of each half
+constexpr int kInferThreads = 32 * (kInferWarps + 1);  // and one warp that issues copies and MMAs
+constexpr int kHalf = kHid / 2;
+constexpr int kWHalfBytes = kHalf * kHid * 2;    // 64 KB: rows of one half of a 256x256 weight image
+constexpr int kWSlots = 3;
 constexpr int kXBytes = kM * 16 * 2;             // 4 KB: the tile's inputs, K padded to 16
 constexpr int kW1Bytes = kHid * 16 * 2;          // 8 KB: W1 image, 256 x 16
 constexpr int kW5Bytes = 16 * kHid * 2;          // 8 KB: W5 image, 16 (3 used) x 256
-constexpr int kOffSmW = kABytes;
-constexpr int kOffSmX = kOffSmW + kWBytes;
+constexpr int kOffSmX = kWSlots * kWHalfBytes;
 constexpr int kOffSmW1 = kOffSmX + kXBytes;
 constexpr int kOffSmW5 = kOffSmW1 + kW1Bytes;
 constexpr int kOffSmBias = kOffSmW5 + kW5Bytes;              // f32 [4][256]: b1..b4
 constexpr int kOffSmB5 = kOffSmBias + 4 * kHid * 4;          // f32 [4]
-constexpr int kOffSmBar = kOffSmB5 + 16;                     // 2 mbarriers
-constexpr int kOffSmSlot = kOffSmBar + 16;                   // TMEM address
+constexpr int kOffSmBar = kOffSmB5 + 16;
+constexpr int kInferBars = kWSlots + 2 + 2 + 3;  // weights arrived; half done; activations written; inputs, output, end
+constexpr int kOffSmSlot = kOffSmBar + 8 * kInferBars;       // TMEM address
 constexpr int kInferSmem = kOffSmSlot + 16;
 static_assert(kOffSmBar % 8 == 0 && kInferSmem <= 227 * 1024, "shared-memory plan");
-// instruction descriptors: N = 256 (hidden layers) and N = 16 (output layer)
-constexpr uint32_t kIdescN16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(16 >> 3) << 17) |
-                               ((uint32_t)(kM >> 4) << 24);
+// tensor memory: two activation images (BF16 pairs, K = 256 in 128 columns), the accumulator
+constexpr uint32_t kTmemD = 2 * kHalf, kTmemCols = 512;
 
 struct InferArgs {
     const float* x;      // [n][6]
     float* y;            // [n][3]
     long long n;
     int tiles;
-    const bf16* wp[3];   // images of W2, W3, W4 (256 x 256)
+    const bf16* wp[3];   // images of W2, W3, W4 (256 x 256; half h is its rows 128 h .., contiguous)
     const bf16* w1p;     // image of W1 padded to 256 x 16
     const bf16* w5p;     // image of W5 padded to 16 x 256
     const float* params;
@@ -651,18 +655,42 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
     v[0] = __uint_as_float(r0); v[1] = __uint_as_float(r1); v[2] = __uint_as_float(r2); v[3] = __uint_as_float(r3);
 }
 
+// D[tmem] (+)= A[tmem] . B[smem desc]^T: the A operand from tensor memory (lane = row, two BF16 of K per column)
+__device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs a) {
     extern __shared__ __align__(1024) unsigned char sm[];
-    bf16* A = reinterpret_cast<bf16*>(sm);
-    bf16* W = reinterpret_cast<bf16*>(sm + kOffSmW);
     unsigned char* X = sm + kOffSmX;
     float* bs = reinterpret_cast<float*>(sm + kOffSmBias);
     float* b5s = reinterpret_cast<float*>(sm + kOffSmB5);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kOffSmBar);  // [0] weights arrived, [1] MMAs done
+    uint64_t* const wfull = reinterpret_cast<uint64_t*>(sm + kOffSmBar);  // [3] a weight half arrived in its slot
+    uint64_t* const dfull = wfull + kWSlots;                              // [2] the MMAs of a half of D completed
+    uint64_t* const aready = dfull + 2;  // [2] a half of D was read and its activations written (per epilogue warp)
+    uint64_t* const xready = aready + 2;  // the tile's inputs are in X and the previous output was read
+    uint64_t* const yfull = xready + 1;   // the output layer's MMAs completed
+    uint64_t* const drained = yfull + 1;  // every MMA issued has completed
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kOffSmSlot);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quarter = warp & 3, cgroup = warp >> 2;  // TMEM lane quarter, group of 64 columns
-    const int r = quarter * 32 + lane;  // this thread's row of the tile (and TMEM lane)
     {
         const uint4* s1 = reinterpret_cast<const uint4*>(a.w1p);
         const uint4* s5 = reinterpret_cast<const uint4*>(a.w5p);
@@ -674,86 +702,104 @@ __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs a
     for (int i = tid; i < 4 * kHid; i += kInferThreads) bs[i] = a.params[off_b(1 + i / kHid) + i % kHid];
     if (tid < kOut) b5s[tid] = a.params[kOffB5 + tid];
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int i = 0; i < kWSlots; ++i) mbar_init(&wfull[i], 1);
+        for (int h = 0; h < 2; ++h) {
+            mbar_init(&dfull[h], 1);
+            mbar_init(&aready[h], kInferWarps);
+        }
+        mbar_init(xready, 4);  // the four warps that hold column group 0
+        mbar_init(yfull, 1);
+        mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(tslot, 256);
+    if (warp == 0) tmem_alloc(tslot, kTmemCols);
+    fence_proxy_async();  // the weight images written above
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
-    const uint32_t sA = smem_u32(A), sW = smem_u32(W), sX = smem_u32(X);
-    const uint32_t sW1 = smem_u32(sm + kOffSmW1), sW5 = smem_u32(sm + kOffSmW5);
-    unsigned wphase = 0, mphase = 0;
-    bool w_pending = false;  // thread 0: a weight copy was issued and not yet waited for
-    if (tid == 0 && (int)blockIdx.x < a.tiles) {
-        bulk_load(W, a.wp[0], kWBytes, &bar[0]);
-        w_pending = true;
-    }
-    // MMAs of one layer by thread 0, then every thread waits for their completion (bounded)
-    auto run_mma = [&](int kind) -> bool {
-        bool issued = true;
-        if (tid == 0) {
-            if (kind == 1) {  // 256x256 layer: needs its weight image
-                issued = mbar_wait(&bar[0], wphase & 1u, a.err, 3);
-                w_pending = !issued;
-            }
-            if (issued) {
+    const int my_tiles = (int)blockIdx.x < a.tiles ? (a.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    if (warp == kInferWarps) {
+        // ---- copies and MMAs (one thread) ----
+        if (lane == 0) {
+            const uint32_t sW = smem_u32(sm), sX = smem_u32(X);
+            const uint32_t sW1 = smem_u32(sm + kOffSmW1), sW5 = smem_u32(sm + kOffSmW5);
+            const int halves = 6 * my_tiles;  // weight halves in the order they are used
+            int loaded = 0, used = 0;
+            auto refill = [&]() {
+                if (loaded >= halves) return;
+                const int i = loaded % 6, slot = loaded % kWSlots;
+                bulk_load(sm + slot * kWHalfBytes, a.wp[i >> 1] + (size_t)(i & 1) * kHalf * kHid, kWHalfBytes, &wfull[slot]);
+                ++loaded;
+            };
+            for (int i = 0; i < kWSlots; ++i) refill();
+            unsigned dphase = 0, aphase = 0;  // completed phases of dfull (both halves alike) and of aready
+            bool ok = true;
+            for (int t = 0; t < my_tiles && ok; ++t) {
+                if (!(ok = mbar_wait(xready, t & 1, a.err, 4))) break;
                 tc_fence_after();
-                if (kind == 0) {
-                    mma_bf16(tmem, smem_desc(sX, 128, 256), smem_desc(sW1, 128, 256), kIdesc, 0u);
-                } else {
-                    const uint32_t b0 = kind == 1 ? sW : sW5;
-                    const uint32_t idesc = kind == 1 ? kIdesc : kIdescN16;
-#pragma unroll
-                    for (int kk = 0; kk < kHid / 16; ++kk)
-                        mma_bf16(tmem, smem_desc(sA + kk * 256, 128, 4096), smem_desc(b0 + kk * 256, 128, 4096),
-                                 idesc, kk > 0 ? 1u : 0u);
+                for (int h = 0; h < 2; ++h) {  // layer 1: K = 16, inputs from shared memory
+                    mma_bf16(tmem + kTmemD + h * kHalf, smem_desc(sX, 128, 256), smem_desc(sW1 + h * 4096, 128, 256),
+                             idesc_of(kHalf), 0u);
+                    mma_commit(&dfull[h]);
                 }
-                mma_commit(&bar[1]);
-            }
-        }
-        if (kind == 1) wphase++;
-        if (!__syncthreads_and(issued)) return false;
-        const bool done = mbar_wait(&bar[1], mphase & 1u, a.err, 4);
-        mphase++;
-        return __syncthreads_and(done);
-    };
-    // bias + SiLU of this thread's 64 columns of the accumulator row into the next A image
-    auto hidden_epilogue = [&](const float* bias) {
-        tc_fence_after();
-#pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-            const int j0 = cgroup * 64 + c * 32;
-            float v[32];
-            tmem_ld32(tlane + (uint32_t)j0, v);
+                ++dphase;
+                for (int l = 0; l < 3 && ok; ++l) {
+                    const uint32_t act = tmem + (l & 1) * kHalf;  // activations of the previous layer
+                    for (int h = 0; h < 2 && ok; ++h) {
+                        const int slot = used % kWSlots;
+                        if (!(ok = mbar_wait(&wfull[slot], (used / kWSlots) & 1, a.err, 3))) break;
+                        const uint32_t w = sW + slot * kWHalfBytes, d = tmem + kTmemD + h * kHalf;
+                        for (int kh = 0; kh < 2 && ok; ++kh) {
+                            // K half kh needs activation half kh; the accumulator half h was read when both are there
+                            if (h == 0) {
+                                if (!(ok = mbar_wait(&aready[kh], aphase & 1, a.err, 5))) break;
+                                tc_fence_after();
+                            }
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float4 b0 = *reinterpret_cast<const float4*>(bias + j0 + 8 * q);
-                const float4 b1 = *reinterpret_cast<const float4*>(bias + j0 + 8 * q + 4);
-                const float* e = v + 8 * q;
-                uint4 o;
-                o.x = pack_bf16x2(silu_tanh(e[0] + b0.x), silu_tanh(e[1] + b0.y));
-                o.y = pack_bf16x2(silu_tanh(e[2] + b0.z), silu_tanh(e[3] + b0.w));
-                o.z = pack_bf16x2(silu_tanh(e[4] + b1.x), silu_tanh(e[5] + b1.y));
-                o.w = pack_bf16x2(silu_tanh(e[6] + b1.z), silu_tanh(e[7] + b1.w));
-                *reinterpret_cast<uint4*>(A + img_idx(r, j0 + 8 * q)) = o;
-            }
-        }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-    };
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x) {
-        const long long row = (long long)tile * kM + r;
-        const bool valid = row < a.n;
-        if (cgroup == 0) {  // the tile's inputs as a 128 x 16 A image (K 6..15 zero)
-            float xv[kIn];
+                            for (int kk = 8 * kh; kk < 8 * kh + 8; ++kk)
+                                mma_bf16_ts(d, act + kk * 8, smem_desc(w + kk * 256, 128, 4096), idesc_of(kHalf),
+                                            kk > 0 ? 1u : 0u);
+                        }
+                        if (ok) mma_commit(&dfull[h]);
+                        ++used;
+                    }
+                    if (!ok) break;
+                    ++aphase;
+                    for (int h = 0; h < 2 && ok; ++h) {  // a half's MMAs completed: its slot takes the next half in line
+                        ok = mbar_wait(&dfull[h], dphase & 1, a.err, 6);
+                        if (ok) refill();
+                    }
+                    ++dphase;
+                }
+                if (!ok) break;
+                for (int kh = 0; kh < 2 && ok; ++kh) ok = mbar_wait(&aready[kh], aphase & 1, a.err, 5);
+                if (!ok) break;
+                ++aphase;
+                tc_fence_after();
 #pragma unroll
-            for (int i = 0; i < kIn; ++i) xv[i] = valid ? a.x[row * kIn + i] : 0.0f;
+                for (int kk = 0; kk < kHid / 16; ++kk)
+                    mma_bf16_ts(tmem + kTmemD, tmem + kHalf + kk * 8, smem_desc(sW5 + kk * 256, 128, 4096), idesc_of(16),
+                                kk > 0 ? 1u : 0u);
+                mma_commit(yfull);
+            }
+            // MMAs and (only after a failed wait) weight copies in flight must end before the CTA leaves
+            mma_commit(drained);
+            (void)mbar_wait(drained, 0, a.err, 10);
+            for (; used < loaded; ++used) (void)mbar_wait(&wfull[used % kWSlots], (used / kWSlots) & 1, a.err, 7);
+        }
+    } else {
+        // ---- inputs, epilogues, outputs ----
+        const int quarter = warp & 3, cgroup = warp >> 2;
+        const int r = quarter * 32 + lane;  // this thread's row of the tile (and TMEM lane)
+        const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
+        float xv[kIn];
+        auto fetch = [&](int t) {  // the inputs of this CTA's tile t
+            const long long row = ((long long)blockIdx.x + (long long)t * gridDim.x) * kM + r;
+#pragma unroll
+            for (int i = 0; i < kIn; ++i) xv[i] = t < my_tiles && row < a.n ? a.x[row * kIn + i] : 0.0f;
+        };
+        auto put = [&]() {  // a 128 x 16 A image (K 6..15 zero)
             uint4 lo;
             lo.x = pack_bf16x2(xv[0], xv[1]);
             lo.y = pack_bf16x2(xv[2], xv[3]);
@@ -761,41 +807,60 @@ __global__ void __launch_bounds__(kInferThreads, 1) mlp_infer_kernel(InferArgs a
             lo.w = 0u;
             *reinterpret_cast<uint4*>(X + (r >> 3) * 256 + (r & 7) * 16) = lo;
             *reinterpret_cast<uint4*>(X + (r >> 3) * 256 + 128 + (r & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+            fence_proxy_async();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(xready);
+        };
+        if (cgroup == 0 && my_tiles > 0) {
+            fetch(0);
+            put();
         }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-        if (!(ok = run_mma(0))) break;
-        hidden_epilogue(bs);
-        for (int l = 0; l < 3 && ok; ++l) {
-            if (!(ok = run_mma(1))) break;
-            // the weight buffer is free: bring in the next layer's weights (or the first layer's for the next tile)
-            if (tid == 0) {
-                if (l < 2) { bulk_load(W, a.wp[l + 1], kWBytes, &bar[0]); w_pending = true; }
-                else if (tile + (int)gridDim.x < a.tiles) { bulk_load(W, a.wp[0], kWBytes, &bar[0]); w_pending = true; }
-            }
-            hidden_epilogue(bs + (l + 1) * kHid);
-        }
-        if (!ok) break;
-        if (!(ok = run_mma(2))) break;
-        tc_fence_after();
-        float v[4];
-        if (cgroup == 0) {
-            tmem_ld4(tlane, v);
-            if (valid)
+        bool ok = true;
+        unsigned dphase = 0;
+        for (int t = 0; t < my_tiles && ok; ++t) {
+            if (cgroup == 0) fetch(t + 1);
+            for (int l = 0; l < 4 && ok; ++l) {  // epilogue of hidden layer l + 1 into activation image l & 1
+                for (int h = 0; h < 2; ++h) {
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait(&dfull[h], dphase & 1, a.err, 8)))) break;
+                    tc_fence_after();
+                    const int j0 = h * kHalf + cgroup * 32;
+                    const float* bias = bs + l * kHid + j0;
+                    float v[32];
+                    tmem_ld32(tlane + kTmemD + (uint32_t)j0, v);
+                    uint32_t o[16];
 #pragma unroll
-                for (int k = 0; k < kOut; ++k) a.y[row * kOut + k] = v[k] + b5s[k];
+                    for (int q = 0; q < 8; ++q) {
+                        const float4 b = *reinterpret_cast<const float4*>(bias + 4 * q);
+                        o[2 * q] = pack_bf16x2(silu_tanh(v[4 * q] + b.x), silu_tanh(v[4 * q + 1] + b.y));
+                        o[2 * q + 1] = pack_bf16x2(silu_tanh(v[4 * q + 2] + b.z), silu_tanh(v[4 * q + 3] + b.w));
+                    }
+                    tmem_st16(tlane + (uint32_t)((l & 1) * kHalf + j0 / 2), o);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&aready[h]);
+                }
+                ++dphase;
+            }
+            if (!ok) break;
+            if (cgroup == 0) {
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait(yfull, t & 1, a.err, 9)))) break;
+                tc_fence_after();
+                float v[4];
+                tmem_ld4(tlane + kTmemD, v);
+                const long long row = ((long long)blockIdx.x + (long long)t * gridDim.x) * kM + r;
+                if (row < a.n)
+#pragma unroll
+                    for (int k = 0; k < kOut; ++k) a.y[row * kOut + k] = v[k] + b5s[k];
+                if (t + 1 < my_tiles) put();
+            }
         }
-        tc_fence_before();
-        __syncthreads();
     }
-    // a weight copy still in flight (only after a failed wait) must land before the CTA leaves
-    if (tid == 0 && w_pending) (void)mbar_wait(&bar[0], wphase & 1u, a.err, 5);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, 256);
+        tmem_dealloc(tmem, kTmemCols);
     }
 }
 
