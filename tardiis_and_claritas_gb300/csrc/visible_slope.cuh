@@ -4,8 +4,7 @@
 // whole cost of rough scenes: of ~50 evaluations per slope only the last few decide anything.
 //
 // Here the same bisection runs, with the same midpoints, and a midpoint's comparison is evaluated only where
-// it could go either way. A root estimate (FP32 search, two FP64 Newton steps with the closed-form derivative)
-// and a bound on how far it and an evaluated midpoint can be off give a radius; outside it the sign of the
+// it could go either way. A root estimate (FP32 search, one FP64 Halley step with closed-form derivatives) and a bound on how far it and an evaluated midpoint can be off give a radius; outside it the sign of the
 // comparison follows from monotonicity. The result is therefore the reference's bit for bit (checked over the
 // declared range of both branches against the plain bisection). Where the estimate is not trusted (no
 // convergence, a root next to the switch of formulas at 5) the radius is infinite: every midpoint is evaluated.
@@ -62,10 +61,11 @@ CLR_SLOPE_FN int o_visible_cdf(double slope, double slope_i, double q, double* o
 }
 
 /* Estimate of the root of F(s) = u on the ordinary branch and the radius outside which the sign of the
- * computed F(mid) - u is that of mid - root. F' = exp(-s^2) (slope_i - s) / (sqrt(pi) q) > 0 below slope_i.
- * The computed F is off by at most 2e-14 for slope_i >= -1 (the two terms of n cancel to no less than a
- * quarter of their size there; exp and erfc are good to a few ulps), so F(root +- r) differs from u by more
- * than both evaluations' error when r = 4e-14 / F', with the curvature over r negligible by the checks. */
+ * computed F(mid) - u is that of mid - root. F' = exp(-s^2) (slope_i - s) / (sqrt(pi) q) > 0 below slope_i and
+ * F''/F' = -2 s - 1/(slope_i - s). The two terms of n are good to a few ulps each (exp 1, erfc 5) and no larger than
+ * those of q, whose absolute sum over q is `spread` (1 for slope_i >= 0, under 8 down to -1): the computed F is off
+ * by less than 1e-15 spread. F(root +- r) differs from u by more than the errors of both evaluations when
+ * r = 8e-15 spread / F', with the curvature over r negligible by the checks. */
 CLR_SLOPE_FN void o_visible_root(double slope_i, double q, double u, double* root, double* radius) {
     *root = 0.0;
     *radius = HUGE_VAL;
@@ -82,25 +82,29 @@ CLR_SLOPE_FN void o_visible_root(double slope_i, double q, double u, double* roo
         s = nx;
     }
     const double K = 0.28209479177387814347403972578038629, SQRT_PI = 1.77245385090551602729816748334114518;
-    double t = (double)s, step = 1.0, p = 0.0;
-    for (int it = 0; it < 4; ++it) {  // two steps, a third or fourth only where FP32 left a poor start
+    double t = (double)s, step = 1.0, p = 0.0, bend = 0.0;
+    for (int it = 0; it < 4; ++it) {  // one step, more only where FP32 left a poor start
         if (!(t < slope_i)) return;
-        const double e = exp(-t * t);
-        p = e * (slope_i - t) / (SQRT_PI * q);
+        const double e = exp(-t * t), room = slope_i - t;
+        p = e * room / (SQRT_PI * q);
         if (!(p > 0.0)) return;
-        step = ((K * e + 0.5 * slope_i * erfc(-t)) / q - u) / p;
+        const double newton = ((K * e + 0.5 * slope_i * erfc(-t)) / q - u) / p;
+        bend = fabs(t) + 1.0 / room;
+        step = newton / (1.0 + newton * (t + 0.5 / room));
         t -= step;
-        if (fabs(step) <= 1.0e-8 * fmin(1.0, slope_i - t)) break;
+        // third order: what is left is below (step bend)^2 step
+        if (fabs(step) * bend <= 1.0e-5) break;
     }
-    const double room = slope_i - t;
-    if (!(room > 0.0) || !(fabs(step) <= 1.0e-8 * fmin(1.0, room)) || !(fabs(t) < 8.0)) return;
-    const double r = 4.0e-14 / p + 1.0e-15;
+    const double room = slope_i - t, spread = slope_i >= 0.0 ? 1.0 : 8.0;
+    if (!(room > 0.0) || !(fabs(step) * bend <= 1.0e-5) || !(fabs(t) < 8.0)) return;
+    const double r = 8.0e-15 * spread / p + 4.0 * (step * bend) * (step * bend) * fabs(step) + 1.0e-15;
     if (!(r <= 1.0e-3 * room) || !(r <= 1.0e-4)) return;
     *root = t;
     *radius = r;
 }
 
-/* The same on the tail branch (x = -slope_i > 1): the root of lr(t) = log(u), lr' = -2 t / C(t), decreasing.
+/* The same on the tail branch (x = -slope_i > 1): the root of lr(t) = log(u), lr' = -2 t / C(t), decreasing, and
+ * lr''/lr' = 1/t - 2 y + 2 t / C with y = x + t.
  * The computed lr is noisy through 1 - y sqrt(pi) erfcx(y): exp(y^2) carries y^2 ulps and the difference is as
  * small as 0.019 at y = 5. Above 5 the asymptotic series is smooth (its own truncation error moves the root
  * but not the order of the values), so only the two sides of 5 may not be compared through one estimate. */
@@ -129,22 +133,27 @@ CLR_SLOPE_FN void o_tail_root(double x, double Bx, double target, double hi0, do
         if (!(nx > lo && nx < hi)) nx = 0.5f * (lo + hi);
         t = nx;
     }
-    double s = (double)t, step = 1.0, C = 1.0;
+    double s = (double)t, step = 1.0, C = 1.0, bend = 0.0;
+    bool enough = false;
     for (int it = 0; it < 4; ++it) {
         if (!(s > 0.0)) return;
         const double y = x + s, By = o_tail_B(y);
         if (!(By > 0.0)) return;
         C = s / y + (x / y) * By;
-        step = (-(2.0 * x * s + s * s) + log(C / Bx) - target) * C / (2.0 * s);
+        const double newton = (-(2.0 * x * s + s * s) + log(C / Bx) - target) * C / (2.0 * s);  // added
+        bend = 1.0 / s + 2.0 * y + 2.0 * s / C;
+        step = newton / (1.0 + newton * (0.5 / s - y + s / C));
         s += step;
-        if (fabs(step) <= 1.0e-8 * s) break;
+        // above 5 the derivatives are those of the whole function, 2e-6 off the cut series': a second step
+        enough = fabs(step) * bend <= (x + s < 4.99 ? 1.0e-5 : 1.0e-9);
+        if (enough) break;
     }
-    if (!(s > 0.0) || !(fabs(step) <= 1.0e-7 * s)) return;
+    if (!(s > 0.0) || !enough) return;
     const double y = x + s;
     if (fabs(y - 5.0) < 1.0e-2) return;
     // noise of lr through C (relative error of B's difference below 5, a few ulps above), and of the sum
-    const double eps = (y < 5.0 ? (1.0e-15 * y * y + 4.0e-15) / C : 2.0e-14) + 4.0e-14;
-    const double r = 4.0 * eps * C / (2.0 * s) + 1.0e-15 * s;
+    const double eps = (y < 5.0 ? (1.0e-15 * y * y + 4.0e-15) / C : 2.0e-14) + 2.0e-14;
+    const double r = 4.0 * eps * C / (2.0 * s) + 4.0 * (step * bend) * (step * bend) * fabs(step) + 1.0e-15 * s;
     if (!(r <= 1.0e-4 * s)) return;
     *root = s;
     *radius = r;
