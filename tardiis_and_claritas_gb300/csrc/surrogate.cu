@@ -147,7 +147,7 @@ constexpr int kStageA = kM * kKC * 2;           // 16 KB
 constexpr int kStageB = kNT * kKC * 2;          // 8 KB
 constexpr int kGemmSmem = kStages * (kStageA + kStageB) + 64;  // stages, barriers, TMEM address
 
-enum Epi : int { EPI_STORE_F32 = 0, EPI_FWD = 1, EPI_BWD = 2, EPI_ADD_F32 = 3 };
+enum Epi : int { EPI_STORE_F32 = 0, EPI_FWD = 1, EPI_BWD = 2 };
 
 struct GemmArgs {
     const bf16* A;           // [M][lda], K contiguous
@@ -157,8 +157,9 @@ struct GemmArgs {
     int M, K, k_split;       // K and k_split multiples of 64; CTA y takes K columns [y*k_split, +k_split)
     const float* bias;       // [256] (EPI_FWD)
     const float* zin;        // [M][256] saved pre-activations (EPI_BWD)
-    float* out_f32;          // [M][ldo]: result (STORE, ADD) or pre-activation z (FWD)
+    float* out_f32;          // [M][ldo]: result (STORE) or pre-activation z (FWD)
     long long ldo;
+    long long part;          // STORE: CTA y's share of K goes to out_f32 + y * part
     bf16* out_bf16;          // [M][256]: silu(z) (FWD) or dz (BWD)
     bf16* out_bf16_t;        // [256][ldt]: transposed copy (FWD, BWD)
     long long ldt;
@@ -263,16 +264,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch ba
         tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * (warp >> 2)), v);
         if (m < g.M) {
             if constexpr (EPI == EPI_STORE_F32) {
-                float4* o = reinterpret_cast<float4*>(g.out_f32 + (long long)m * g.ldo + j0);
+                float4* o = reinterpret_cast<float4*>(g.out_f32 + blockIdx.y * g.part + (long long)m * g.ldo + j0);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            } else if constexpr (EPI == EPI_ADD_F32) {
-                float* o = g.out_f32 + (long long)m * g.ldo + j0;
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o + 4 * i), "f"(v[4 * i]),
-                                 "f"(v[4 * i + 1]), "f"(v[4 * i + 2]), "f"(v[4 * i + 3])
-                                 : "memory");
             } else if constexpr (EPI == EPI_FWD) {
                 __align__(16) bf16 hb[32];
 #pragma unroll
@@ -320,7 +314,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch ba
 // stream capture).
 static cudaError_t set_gemm_attributes() {
     const void* fns[] = {(const void*)umma_gemm_kernel<EPI_STORE_F32>, (const void*)umma_gemm_kernel<EPI_FWD>,
-                         (const void*)umma_gemm_kernel<EPI_BWD>, (const void*)umma_gemm_kernel<EPI_ADD_F32>};
+                         (const void*)umma_gemm_kernel<EPI_BWD>};
     for (const void* f : fns) {
         cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
         if (e != cudaSuccess) return e;
@@ -468,13 +462,47 @@ __global__ void __launch_bounds__(256) head_kernel(StepArgs* a, const bf16* __re
 // output gradients are staged in shared memory (a thread that loads them row by row waits for memory at each):
 //   db_l[j] = sum_r dz_l[r][j] (l = 1..4), with it for l = 1 dW1[j][i] = sum_r dz1[r][j] x[r][i];
 //   dW5[k][j] = sum_r dy[r][k] h4[r][j]; and one thread for db5[k] = sum_r dy[r][k].
+// A block's sums go to its own row of partial sums (`parts`); they are added in the rows' order where the gradient is
+// used, so a step does not depend on which block ends first (added with atomics, two runs of an epoch differed by up
+// to 5e-5 of the largest weight, Adam's first steps being the signs of the gradients).
+constexpr int kHiddenW = 3 * kHid * kHid, kSmallParams = (int)kParams - kHiddenW;
+constexpr int kWeightRows = 512;  // batch rows of a partial sum of W2..W4
+struct GradParts {
+    const float* hidden;  // [n_hidden][3][256][256]: W2, W3, W4
+    const float* rest;    // [n_rest][kSmallParams]: the other parameters in their order
+    int n_hidden, n_rest;
+};
+__host__ __device__ constexpr int rest_index(int p) {
+    return p - kHid * kHid * ((p >= (int)off_b(2)) + (p >= (int)off_b(3)) + (p >= (int)off_b(4)));
+}
+static_assert(rest_index((int)kParams - 1) == kSmallParams - 1, "the parameters outside W2..W4, gap-free");
+__device__ __forceinline__ float grad_of(const GradParts& G, int p) {
+    const float* src = G.rest + rest_index(p);
+    int rows = G.n_rest;
+    long long stride = kSmallParams;
+#pragma unroll
+    for (int l = 2; l <= 4; ++l)
+        if (p >= (int)off_w(l) && p < (int)off_b(l)) {
+            src = G.hidden + (l - 2) * kHid * kHid + (p - (int)off_w(l));
+            rows = G.n_hidden;
+            stride = kHiddenW;
+        }
+    float g = 0.0f;
+#pragma unroll 4
+    for (int i = 0; i < rows; ++i) g += src[i * stride];
+    return g;
+}
+__global__ void sum_grads_kernel(GradParts G, float* grads) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < (int)kParams) grads[p] = grad_of(G, p);
+}
 constexpr int kSmallUnits = 5 * kHid + 1;
 constexpr int kSmallRows = 256;
 constexpr int kSmallThreads = 64;
 __global__ void __launch_bounds__(kSmallThreads) small_grads_kernel(const bf16* const* __restrict__ dzt,
                                                                     const bf16* __restrict__ h4t, long long ldt,
                                                                     const float* __restrict__ xb,
-                                                                    const float* __restrict__ dy, int n, float* grads) {
+                                                                    const float* __restrict__ dy, int n, float* parts) {
     __shared__ float xs[kSmallRows * kIn], ds[kSmallRows * kOut];
     const int r0 = blockIdx.y * kSmallRows, rows = min(n - r0, kSmallRows);  // a multiple of 128
     const int unit = blockIdx.x * kSmallThreads + threadIdx.x;
@@ -513,14 +541,15 @@ __global__ void __launch_bounds__(kSmallThreads) small_grads_kernel(const bf16* 
             }
         }
     }
+    float* const out = parts + (long long)blockIdx.y * kSmallParams;
     if (what < 4) {
-        atomicAdd(grads + off_b(what + 1) + j, s[kIn]);
+        out[rest_index((int)off_b(what + 1) + j)] = s[kIn];
         if (what == 0)
 #pragma unroll
-            for (int i = 0; i < kIn; ++i) atomicAdd(grads + kOffW1 + j * kIn + i, s[i]);
+            for (int i = 0; i < kIn; ++i) out[rest_index((int)kOffW1 + j * kIn + i)] = s[i];
     } else {
 #pragma unroll
-        for (int k = 0; k < kOut; ++k) atomicAdd(grads + (what == 4 ? kOffW5 + k * kHid + j : kOffB5 + k), s[k]);
+        for (int k = 0; k < kOut; ++k) out[rest_index((int)(what == 4 ? kOffW5 + k * kHid + j : kOffB5 + k))] = s[k];
     }
 }
 
@@ -566,20 +595,19 @@ __global__ void pack_kernel(const float* __restrict__ params, PackArgs pa) {
 
 // Adam (bias-corrected) on every parameter, then the gradient is cleared and the BF16 copies refreshed. hp: per
 // step of the call the learning rate and the two bias corrections.
-__global__ void adam_kernel(float* params, float* grads, float* m1, float* m2, const StepArgs* __restrict__ step,
+__global__ void adam_kernel(float* params, GradParts G, float* m1, float* m2, const StepArgs* __restrict__ step,
                             const float4* __restrict__ hp, PackArgs pa) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (int)kParams) return;
     const float4 h = hp[step->step - 1];
     const float lr = h.x, c1 = h.y, c2 = h.z;
-    const float g = grads[p];
+    const float g = grad_of(G, p);
     const float a = 0.9f * m1[p] + 0.1f * g;
     const float b = 0.999f * m2[p] + 0.001f * g * g;
     m1[p] = a;
     m2[p] = b;
     const float v = params[p] - lr * (a / c1) / (sqrtf(b / c2) + 1e-8f);
     params[p] = v;
-    grads[p] = 0.0f;
     pack_one(pa, p, v);
 }
 
@@ -877,6 +905,7 @@ struct clr_mlp {
     std::string err;
     std::vector<void*> allocs;
     float *params = nullptr, *grads = nullptr, *m1 = nullptr, *m2 = nullptr;
+    float *hidden_parts = nullptr, *rest_parts = nullptr;  // partial gradients of a step (GradParts)
     PackArgs pa{};
     float* z[5] = {};          // [cap][256] pre-activations of hidden layers 1..4
     bf16* h[5] = {};           // [cap][256] activations
@@ -940,7 +969,7 @@ static cudaError_t forward_rows(clr_mlp* m, int n, cudaStream_t st) {
     return cudaSuccess;
 }
 
-// Backward pass of the n rows of the last forward (targets in tb): gradients accumulate into grads.
+// Backward pass of the n rows of the last forward (targets in tb): gradients as partial sums (grad_parts).
 static cudaError_t backward_rows(clr_mlp* m, int n, cudaStream_t st) {
     head_kernel<<<n / kThinRows, 256, 0, st>>>(m->d_step, m->h[4], m->z[4], n, m->pa.w[5], m->params + kOffB5, m->tb,
                                                m->wb, m->dy, m->dz[4], m->dzt[4], m->cap, m->loss);
@@ -959,19 +988,22 @@ static cudaError_t backward_rows(clr_mlp* m, int n, cudaStream_t st) {
     if ((e = cudaEventRecord(m->fork, st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(m->side, m->fork, 0)) != cudaSuccess) return e;
     small_grads_kernel<<<dim3((kSmallUnits + kSmallThreads - 1) / kSmallThreads, (n + kSmallRows - 1) / kSmallRows),
-                         kSmallThreads, 0, m->side>>>(m->d_dzt, m->ht[4], m->cap, m->xb, m->dy, n, m->grads);
+                         kSmallThreads, 0, m->side>>>(m->d_dzt, m->ht[4], m->cap, m->xb, m->dy, n, m->rest_parts);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = cudaEventRecord(m->join, m->side)) != cudaSuccess) return e;
-    const int ksplit = 512;
     GemmBatch b{};
     for (int l = 2; l <= 4; ++l) {  // dW_l = dz_l^T . h_{l-1}, split over the batch, the three layers in one launch
         GemmArgs& g = b.g[l - 2];
         g.A = m->dzt[l]; g.lda = m->cap; g.B = m->ht[l - 1]; g.ldb = m->cap;
-        g.M = kHid; g.K = n; g.k_split = ksplit;
-        g.out_f32 = m->grads + off_w(l); g.ldo = kHid; g.err = m->d_err;
+        g.M = kHid; g.K = n; g.k_split = kWeightRows;
+        g.out_f32 = m->hidden_parts + (l - 2) * kHid * kHid; g.ldo = kHid; g.part = kHiddenW; g.err = m->d_err;
     }
-    if ((e = launch_gemm<EPI_ADD_F32>(b, kGemmBatch, (n + ksplit - 1) / ksplit, st)) != cudaSuccess) return e;
+    if ((e = launch_gemm<EPI_STORE_F32>(b, kGemmBatch, (n + kWeightRows - 1) / kWeightRows, st)) != cudaSuccess) return e;
     return cudaStreamWaitEvent(st, m->join, 0);
+}
+
+static GradParts grad_parts(const clr_mlp* m, int n) {
+    return {m->hidden_parts, m->rest_parts, (n + kWeightRows - 1) / kWeightRows, (n + kSmallRows - 1) / kSmallRows};
 }
 
 static int check_dev(clr_mlp* m) {
@@ -1018,6 +1050,9 @@ int clr_mlp_create(clr_mlp** out, int device, int max_batch, uint64_t seed) {
             MCU(cudaMemset(m->pa.wp[l], 0, (size_t)kHid * 16 * sizeof(bf16)));
         }
     }
+    const GradParts most = grad_parts(m, m->cap);
+    MCU(F(&m->hidden_parts, (size_t)most.n_hidden * kHiddenW));
+    MCU(F(&m->rest_parts, (size_t)most.n_rest * kSmallParams));
     const size_t act = (size_t)m->cap * kHid;
     for (int l = 1; l <= 4; ++l) {
         MCU(F(&m->z[l], act)); MCU(H(&m->h[l], act)); MCU(H(&m->ht[l], act));
@@ -1031,7 +1066,6 @@ int clr_mlp_create(clr_mlp** out, int device, int max_batch, uint64_t seed) {
     const bf16* dzt[4] = {m->dzt[1], m->dzt[2], m->dzt[3], m->dzt[4]};
     MCU(cudaMemcpy(m->d_dzt, dzt, sizeof dzt, cudaMemcpyHostToDevice));
     MCU(cudaMemset(m->d_err, 0, sizeof(int)));
-    MCU(cudaMemset(m->grads, 0, kParams * sizeof(float)));
     MCU(cudaMemset(m->m1, 0, kParams * sizeof(float)));
     MCU(cudaMemset(m->m2, 0, kParams * sizeof(float)));
     // initial weights and biases uniform in +-1/sqrt(fan_in) from a seeded host generator
@@ -1119,7 +1153,6 @@ int clr_mlp_gradients(clr_mlp* m, const float* d_x, const float* d_t, int64_t n,
         return mfail(m, CLR_ERR_INVALID_ARGUMENT, "clr_mlp_gradients: n must be a multiple of 128 up to max_batch");
     MCU(cudaSetDevice(m->device));
     cudaStream_t st = m->stream;
-    MCU(cudaMemsetAsync(m->grads, 0, kParams * sizeof(float), st));
     MCU(cudaMemsetAsync(m->loss, 0, sizeof(float), st));
     const StepArgs args = {d_x, d_t, m->d_w, nullptr, 0};
     MCU(cudaMemcpyAsync(m->d_step, &args, sizeof args, cudaMemcpyHostToDevice, st));
@@ -1127,8 +1160,11 @@ int clr_mlp_gradients(clr_mlp* m, const float* d_x, const float* d_t, int64_t n,
     MCU(backward_rows(m, (int)n, st));
     float ls = 0.0f;
     MCU(cudaMemcpyAsync(&ls, m->loss, sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (grads_host) MCU(cudaMemcpyAsync(grads_host, m->grads, kParams * sizeof(float), cudaMemcpyDeviceToHost, st));
-    MCU(cudaMemsetAsync(m->grads, 0, kParams * sizeof(float), st));
+    if (grads_host) {
+        sum_grads_kernel<<<(int)((kParams + 255) / 256), 256, 0, st>>>(grad_parts(m, (int)n), m->grads);
+        MCU(cudaGetLastError());
+        MCU(cudaMemcpyAsync(grads_host, m->grads, kParams * sizeof(float), cudaMemcpyDeviceToHost, st));
+    }
     int rc = check_dev(m);
     if (rc != CLR_OK) return rc;
     if (loss) *loss = ls / (3.0f * (float)n);
@@ -1150,7 +1186,7 @@ static int build_step_graph(clr_mlp* m, int n) {
     cudaError_t e = forward_rows(m, n, st);
     if (e == cudaSuccess) e = backward_rows(m, n, st);
     if (e == cudaSuccess) {
-        adam_kernel<<<(int)((kParams + 255) / 256), 256, 0, st>>>(m->params, m->grads, m->m1, m->m2, m->d_step, m->d_hp,
+        adam_kernel<<<(int)((kParams + 255) / 256), 256, 0, st>>>(m->params, grad_parts(m, n), m->m1, m->m2, m->d_step, m->d_hp,
                                                                   m->pa);
         e = cudaGetLastError();
     }

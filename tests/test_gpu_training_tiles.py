@@ -93,3 +93,22 @@ def test_training_steps_follow_their_inputs(torch_cuda):
         assert np.linalg.norm(a - b) < 1e-3 * np.linalg.norm(a - before) + 1e-7 * np.linalg.norm(a)
     for net in nets:
         net.close()
+
+
+@pytest.mark.parametrize("n", [128, 640, 1024])
+def test_gradients_are_the_same_bits_in_every_run(torch_cuda, n):
+    """Partial sums are added in a fixed order, and those of a larger batch before leave nothing behind."""
+    torch = torch_cuda
+    from tardiis_and_claritas_gb300 import lib as L
+    rng = np.random.default_rng(3)
+    x = torch.from_numpy(rng.normal(size=(1024, 6)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.normal(size=(1024, 3)).astype(np.float32)).cuda()
+    got = []
+    for before in (0, 1024, n):
+        net = L.Network(0, max_batch=1024, seed=1)
+        net.set_params(M.init_params(11))
+        if before:
+            net.gradients(x.data_ptr(), t.data_ptr(), before)
+        got.append(net.gradients(x.data_ptr(), t.data_ptr(), n)[1])
+    np.testing.assert_array_equal(got[0], got[1])
+    np.testing.assert_array_equal(got[0], got[2])
