@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(256) head_kernel(StepArgs* a, const bf16* __re
                                                    int n, const bf16* __restrict__ w5, const float* __restrict__ b5,
                                                    const float* __restrict__ tb, const float* __restrict__ wb, float* dy,
                                                    bf16* dz4, bf16* dz4t, long long ldt, float* loss_sum) {
-    __shared__ bf16 tile[kThinRows][kHid + 8];
+    __shared__ __align__(16) bf16 tile[kThinRows][kHid + 8];  // stored 16 bytes at a time
     __shared__ float block_loss[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = blockIdx.x * kThinRows;
     if (blockIdx.x == 0 && threadIdx.x == 0) a->step += 1;
