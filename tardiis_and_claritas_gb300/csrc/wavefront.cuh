@@ -72,9 +72,9 @@ constexpr int kCondInline = 8;
 constexpr int kCondBudget = 512;
 // trials per COND visit when a whole warp runs them (counter-based stream): 32 warp steps
 constexpr int kCondWarpBudget = 1024;
-// trials a lane runs on its own before the rest of its closure goes across the warp (diagnostic COND stage and
-// tail kernel, counter-based stream): most closures of a scattered target end in one or two, an absorbed
-// target of a weakly absorbing particle takes hundreds
+// trials a lane runs on its own before the rest of its closure goes across the warp (diagnostic COND stage,
+// counter-based stream): most closures of a scattered target end in one or two, an absorbed target of a weakly
+// absorbing particle takes hundreds. The tail kernel has no such second part: its lanes take kCondBudget a visit.
 constexpr int kCondAlone = 12;
 
 template <class Mode>
@@ -374,8 +374,8 @@ __global__ void __launch_bounds__(kWaveThreads) wave_gen_kernel(WaveLaunch w) {
 // ---------------- generic stage kernel (ENTRY, FLIGHT and the event handlers) ----------------
 // kLight: the water flights carry the diagnostic hooks, light history and particle-event provenance (a
 // separate FLIGHT kernel, used only when a diagnostic is on, keeps them out of the production kernel).
-// pv: the photon's provenance state, or null when provenance is not counted.
-template <class Mode, int Q, bool kLight = true>
+// pv: the photon's provenance state, or null when provenance is not counted. kTrials: closure trials of a COND visit.
+template <class Mode, int Q, bool kLight = true, int kTrials = kCondBudget>
 __device__ __forceinline__ int wave_stage_body(const WaveLaunch& w, const DevScene& D, Ray& r,
                                                typename Mode::Lane& L, SlotMeta& m,
                                                unsigned long long* cstats, uint4* pv) {
@@ -431,8 +431,7 @@ __device__ __forceinline__ int wave_stage_body(const WaveLaunch& w, const DevSce
             v = closure_visit(D, r, L.optics(), cstats, m.pidx, CK_GEOM, &cs, kCondInline);
         } else {
             cs.started = m.cond_started; cs.trial = m.cond_trial; cs.target = m.cond_target;
-            v = closure_visit(D, r, L.optics(), cstats, m.pidx, m.cond_kind, &cs,
-                              kCounterStream<typename Mode::Stream> ? kCondAlone : kCondBudget);
+            v = closure_visit(D, r, L.optics(), cstats, m.pidx, m.cond_kind, &cs, kTrials);
         }
         if (v == 2) {
             m.cond_started = cs.started; m.cond_trial = cs.trial; m.cond_target = cs.target;
@@ -645,7 +644,7 @@ __global__ void __launch_bounds__(kWaveThreads, 1) wave_cond_diag_kernel(WaveLau
             uint4 pvv;
             uint4* pv = nullptr;
             if (w.prov) { pvv = w.prov[slot]; pv = &pvv; }
-            dest = wave_stage_body<Mode, WQ_COND, true>(w, D, r, L, m, w.tallies[m.sid].c.cstats, pv);
+            dest = wave_stage_body<Mode, WQ_COND, true, kCondAlone>(w, D, r, L, m, w.tallies[m.sid].c.cstats, pv);
             if (pv) w.prov[slot] = pvv;
             pool.ray[slot] = r;
             pool.lane[slot] = L;
