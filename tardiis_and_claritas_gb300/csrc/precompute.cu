@@ -340,6 +340,12 @@ __global__ void __launch_bounds__(32) legendre_table_kernel(const double* __rest
 // Coefficients and the quotients of an order (identical to evaluating them inline) are staged kPdfStage orders at
 // a time.
 constexpr int kPdfManyBins = 608;
+// Without the table (thousands of angles and orders, so warps enough) four bins to a warp share the recurrence: 22
+// operations per bin and order instead of 28 (fast arithmetic 17.5 instead of 22). The line is where that outweighs
+// the longer warps of the largest sizes in both arithmetics (one bin / four bins, ms; 12289 angles in the reference's
+// order, 24001 fast): 141 bins 28.7 / 30.0 and 14.5 / 12.6, 188 bins 38.0 / 36.9 and 19.0 / 15.9, 611 bins 120.5 /
+// 101.1 and 58.5 / 47.5.
+constexpr int kPdfManyBinsNoTable = 160;
 constexpr int kPdfPad = 14 * 1024;  // unused shared memory per block of one bin: 12 blocks per SM, the rest wait, so
                                     // that a partition whose warps end early takes the next (2.78 ms with all resident)
 constexpr int kPdfStage = 64;
@@ -1559,22 +1565,28 @@ cudaError_t enqueue_mie_tables(const double* d, const double* nr, const double* 
     if (hybrid) {
         if (!b.table) theta_grid_kernel<<<(nt + 127) / 128, 128, 0, st>>>(b.theta, b.theta_f, nt);
         else if (b.table_ready && (e = cudaStreamWaitEvent(st, b.table_ready, 0)) != cudaSuccess) return e;
-        const dim3 one((nt + 31) / 32, n), four((nt + 31) / 32, (n + 3) / 4);
         const int pairs = (nt + 1) / 2, pitch = legendre_pitch(nt, fast_pdf);
-        if (fast_pdf) {
-            auto fast = [&](auto kernel, int group, int threads, size_t pad) {
-                kernel<<<dim3((pairs + threads - 1) / threads, (n + group - 1) / group), threads, pad, st>>>(
-                    b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
-            };
-            if (!b.table) fast(phase_pdf_fast_kernel<1, 32, false>, 1, 32, kPdfPad);
-            else if (n < kPdfManyBins) fast(phase_pdf_fast_kernel<1, 32, true>, 1, 32, kPdfPad);
-            else fast(phase_pdf_fast_kernel<4, 128, true>, 4, 128, 0);
-        } else if (!b.table) {
-            phase_pdf_kernel<1, false><<<one, 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, nullptr, 0, b.pdf);
-        } else if (n < kPdfManyBins) {
-            phase_pdf_kernel<1, true><<<one, 32, kPdfPad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
+        const bool many = n >= (b.table ? kPdfManyBins : kPdfManyBinsNoTable);
+        auto ordered = [&](auto kernel, int group, size_t pad) {
+            kernel<<<dim3((nt + 31) / 32, (n + group - 1) / group), 32, pad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab,
+                                                                                   b.table, pitch, b.pdf);
+        };
+        auto fast = [&](auto kernel, int group, int threads, size_t pad) {
+            kernel<<<dim3((pairs + threads - 1) / threads, (n + group - 1) / group), threads, pad, st>>>(
+                b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
+        };
+        if (fast_pdf && many) {
+            if (b.table) fast(phase_pdf_fast_kernel<4, 128, true>, 4, 128, 0);
+            else fast(phase_pdf_fast_kernel<4, 128, false>, 4, 128, 0);
+        } else if (fast_pdf) {
+            if (b.table) fast(phase_pdf_fast_kernel<1, 32, true>, 1, 32, kPdfPad);
+            else fast(phase_pdf_fast_kernel<1, 32, false>, 1, 32, kPdfPad);
+        } else if (many) {
+            if (b.table) ordered(phase_pdf_kernel<4, true>, 4, 0);
+            else ordered(phase_pdf_kernel<4, false>, 4, 0);
         } else {
-            phase_pdf_kernel<4, true><<<four, 32, 0, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
+            if (b.table) ordered(phase_pdf_kernel<1, true>, 1, kPdfPad);
+            else ordered(phase_pdf_kernel<1, false>, 1, kPdfPad);
         }
         const size_t row = nt <= kCdfSmemAngles ? (size_t)nt * sizeof(double) : 0;
         phase_cdf_kernel<<<n, kCdfThreads, row, st>>>(b.theta, b.pdf, nt, n, b.cdf, b.cdf_f, b.err);
