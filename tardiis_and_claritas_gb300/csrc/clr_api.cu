@@ -26,13 +26,13 @@ struct clr_ctx {
     bool scene_set = false, built = false;
     clr_scene_params sp{};
     ParticleBuffers pb{};
-    // the tables of the current scene, carved from one arena that grows to the largest scene built and is kept (55
-    // allocations and releases per build, each of which waits for the device, were 0.6 of a 4.8 ms build), and a
-    // pinned buffer through which they are read back in one copy
+    // the tables of the current scene, carved from one arena that is kept for the next build (55 allocations and
+    // releases per build, each of which waits for the device, were 0.6 of a 4.8 ms build), and a pinned buffer through
+    // which they are read back in one copy; both are given back by one rule (oversized)
     void* build_arena = nullptr;
-    size_t build_arena_bytes = 0;
+    size_t build_arena_bytes = 0, build_arena_need = 0;  // need: of the last build
     void* h_stage = nullptr;
-    size_t h_stage_bytes = 0;
+    size_t h_stage_bytes = 0, h_stage_need = 0;
     // per-run device buffers (single scenario)
     DevScene* d_scene = nullptr;
     long long* d_chunk_begin = nullptr;
@@ -100,6 +100,14 @@ static int fail(clr_ctx* c, int code, const char* fmt, ...) {
     } while (0)
 
 static int run_buffers_ready(clr_ctx* ctx, int n);
+
+// A kept buffer is given back once two uses in a row needed less than a quarter of it, by 64 MB at least: a caller that
+// turned from a large scene to small ones gets the memory back, one that goes to and fro between sizes keeps it (217 MB
+// cost 0.8 ms to release and allocate again, beside builds of 2.4 and 0.2 ms).
+static bool oversized(size_t held, size_t need, size_t before) {
+    const size_t use = std::max(need, before);
+    return held / 4 > use && held - use >= ((size_t)64 << 20);
+}
 
 // Bump allocator over one device arena; with base 0 it only measures.
 struct Arena {
@@ -370,7 +378,9 @@ int clr_build_particles(clr_ctx* ctx, const clr_particle_spec* ps, const clr_sed
         return A.off;
     };
     const size_t need = carve(Arena{});
-    if (need > ctx->build_arena_bytes) {
+    const bool release = oversized(ctx->build_arena_bytes, need, ctx->build_arena_need);
+    ctx->build_arena_need = need;
+    if (need > ctx->build_arena_bytes || release) {
         CU(cudaStreamSynchronize(ctx->stream));
         cudaFree(ctx->build_arena);
         ctx->build_arena = nullptr;
@@ -475,7 +485,9 @@ static int read_physics(clr_ctx* ctx, const ParticleBuffers& pb, clr_particle_ph
     span(o->nstop, pb.nstop, n * sizeof(int));
     if (sum == 0) return CLR_OK;
     if (hi - lo <= 2 * sum + 16384) {
-        if (hi - lo > ctx->h_stage_bytes) {
+        const bool release = oversized(ctx->h_stage_bytes, hi - lo, ctx->h_stage_need);
+        ctx->h_stage_need = hi - lo;
+        if (hi - lo > ctx->h_stage_bytes || release) {
             if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
             ctx->h_stage = nullptr;
             ctx->h_stage_bytes = 0;
