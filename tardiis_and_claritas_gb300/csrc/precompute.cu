@@ -335,19 +335,22 @@ __global__ void __launch_bounds__(32) legendre_table_kernel(const double* __rest
 // pipe (20 operations per bin and order; without the table of pi_n, tau_n 8 more per order; no contraction).
 // A warp issues one FP64 instruction per 64 cycles, so few bins make the largest sizes' warps the longest: with four
 // bins to a warp in blocks of 128 angles, the last blocks of 63 bins ran 4.4 ms where the pipe's work is 1.2 ms.
-// One warp per block, the last bins (usually the largest, with the most orders) first, and kPdfGroup = 1 below
-// kPdfManyBins bins (an even load), 4 above (fewer loads, and enough blocks to even out).
+// One warp per block, the last bins (usually the largest, with the most orders) first, and one bin to a warp: with the
+// table, four bins would only share its loads, which the FP64 pipe hides, and are slower at every size (ms in the
+// reference's order / fast: 640 bins of the sweep workload 11.2 / 3.4 against 14.9 / 4.2 with four, 4096 bins 64.3 /
+// 15.4 against 66.8 / 17.7; 640 bins of 257 angles 3.2 / 1.8 against 4.6 / 2.6).
 // Coefficients and the quotients of an order (identical to evaluating them inline) are staged kPdfStage orders at
 // a time.
-constexpr int kPdfManyBins = 608;
 // Without the table (thousands of angles and orders, so warps enough) four bins to a warp share the recurrence: 22
 // operations per bin and order instead of 28 (fast arithmetic 17.5 instead of 22). The line is where that outweighs
 // the longer warps of the largest sizes in both arithmetics (one bin / four bins, ms; 12289 angles in the reference's
 // order, 24001 fast): 141 bins 28.7 / 30.0 and 14.5 / 12.6, 188 bins 38.0 / 36.9 and 19.0 / 15.9, 611 bins 120.5 /
 // 101.1 and 58.5 / 47.5.
-constexpr int kPdfManyBinsNoTable = 160;
-constexpr int kPdfPad = 14 * 1024;  // unused shared memory per block of one bin: 12 blocks per SM, the rest wait, so
-                                    // that a partition whose warps end early takes the next (2.78 ms with all resident)
+constexpr int kPdfManyBins = 160;
+// Unused shared memory per block of one bin: about a dozen blocks per SM, the rest wait, so that a partition whose warps
+// end early takes the next (282 bins of 1801 angles 5.9 ms, 7.2 with all resident; the fast kernel, whose own 4 KB are
+// nearly the same, 1.8 ms against 2.0 for 141 bins of 2401 angles and within 3 % at most other sizes).
+constexpr int kPdfPad = 14 * 1024;
 constexpr int kPdfStage = 64;
 template <int kPdfGroup, bool kTable>
 __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict__ theta, int nt, int n_particles,
@@ -433,9 +436,8 @@ __global__ void __launch_bounds__(32) phase_pdf_kernel(const double* __restrict_
 // sums over odd and over even orders of a pi_n, b tau_n, a tau_n and b pi_n give S1 and S2 at mu and at
 // -mu: 8 FMAs per (bin, order) for both angles, against about 44 FP64 operations of the reference's order
 // of operations for the two. Tables differ from the reference-order ones by rounding only (tested).
-// pi_n and tau_n come from the table. kPdfFastGroup bins share their loads: 4 where there are many bins and the FP64
-// pipe is the bound, 1 in one-warp blocks, the last bins first, where the largest sizes' warps are (a warp issues one
-// FP64 instruction per 64 cycles; see phase_pdf_kernel).
+// pi_n and tau_n come from the table, for one bin in a one-warp block, the last bins first; many bins without a table
+// share the recurrence, four to a block (both by the rule of phase_pdf_kernel).
 constexpr int kPdfFastChunk = 128;  // orders staged per block
 template <int kPdfFastGroup, int kThreads, bool kTable>
 __global__ void __launch_bounds__(kThreads) phase_pdf_fast_kernel(const double* __restrict__ theta, int nt,
@@ -1566,7 +1568,7 @@ cudaError_t enqueue_mie_tables(const double* d, const double* nr, const double* 
         if (!b.table) theta_grid_kernel<<<(nt + 127) / 128, 128, 0, st>>>(b.theta, b.theta_f, nt);
         else if (b.table_ready && (e = cudaStreamWaitEvent(st, b.table_ready, 0)) != cudaSuccess) return e;
         const int pairs = (nt + 1) / 2, pitch = legendre_pitch(nt, fast_pdf);
-        const bool many = n >= (b.table ? kPdfManyBins : kPdfManyBinsNoTable);
+        const bool many = !b.table && n >= kPdfManyBins;
         auto ordered = [&](auto kernel, int group, size_t pad) {
             kernel<<<dim3((nt + 31) / 32, (n + group - 1) / group), 32, pad, st>>>(b.theta, nt, n, order_cap, b.nstop, b.ab,
                                                                                    b.table, pitch, b.pdf);
@@ -1575,17 +1577,13 @@ cudaError_t enqueue_mie_tables(const double* d, const double* nr, const double* 
             kernel<<<dim3((pairs + threads - 1) / threads, (n + group - 1) / group), threads, pad, st>>>(
                 b.theta, nt, n, order_cap, b.nstop, b.ab, b.table, pitch, b.pdf);
         };
-        if (fast_pdf && many) {
-            if (b.table) fast(phase_pdf_fast_kernel<4, 128, true>, 4, 128, 0);
-            else fast(phase_pdf_fast_kernel<4, 128, false>, 4, 128, 0);
-        } else if (fast_pdf) {
+        if (fast_pdf) {
             if (b.table) fast(phase_pdf_fast_kernel<1, 32, true>, 1, 32, kPdfPad);
+            else if (many) fast(phase_pdf_fast_kernel<4, 128, false>, 4, 128, 0);
             else fast(phase_pdf_fast_kernel<1, 32, false>, 1, 32, kPdfPad);
-        } else if (many) {
-            if (b.table) ordered(phase_pdf_kernel<4, true>, 4, 0);
-            else ordered(phase_pdf_kernel<4, false>, 4, 0);
         } else {
             if (b.table) ordered(phase_pdf_kernel<1, true>, 1, kPdfPad);
+            else if (many) ordered(phase_pdf_kernel<4, false>, 4, 0);
             else ordered(phase_pdf_kernel<1, false>, 1, kPdfPad);
         }
         const size_t row = nt <= kCdfSmemAngles ? (size_t)nt * sizeof(double) : 0;

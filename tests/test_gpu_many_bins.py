@@ -1,9 +1,9 @@
 """GPU: the phase tables of a sweep equal a single scene's at every number of bins.
 
-The phase pdf takes one bin or four to a warp by the number of bins, in both arithmetics, and runs with the table of the
-angular functions or (above 256 MB) without. Every bin has the same operations in the same order in all of them, so
-the tables of a scenario are those of its single build bit for bit: totals below, at and above the lines (608 bins;
-160 without the table), a last group of four with missing bins, and angles that fill neither a warp nor a block.
+The phase pdf takes one bin to a warp or, without the table of the angular functions (above 256 MB of it), four from
+160 bins on, in both arithmetics. Every bin has the same operations in the same order in all of them, so the tables of
+a scenario are those of its single build bit for bit: hundreds of bins with the table, totals below, at and above the
+line without it, a last group of four with missing bins, and angles that fill neither a warp nor a block.
 """
 from __future__ import annotations
 
@@ -42,7 +42,7 @@ def _check(ctx, sizes, n_theta, d_max_um, arithmetic, compare):
 
 
 @pytest.mark.parametrize("arithmetic", [abi.TABLES_REFERENCE, abi.TABLES_FAST])
-@pytest.mark.parametrize("last", [43, 44, 47])  # 607, 608 and 611 bins
+@pytest.mark.parametrize("last", [43, 44, 47])  # 607, 608 and 611 bins: a multiple of four and not
 def test_sweep_tables_equal_single_builds(ctx, arithmetic, last):
     _check(ctx, [47] * 12 + [last], 1801, 60.0, arithmetic, range(13))
 
