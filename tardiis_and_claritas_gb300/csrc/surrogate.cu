@@ -140,12 +140,20 @@ constexpr uint32_t kIdesc = idesc_of(kN);
 // epilogue. A CTA takes 64 of the 256 output columns (64 CTAs for 2048 rows instead of 16), brings its whole
 // K = 256 in with asynchronous copies before the first MMA (four stages of 64), and eight warps share the
 // epilogue, 32 columns each. With 128 x 256 tiles, plain loads two stages deep and four warps a layer took 52 us.
-constexpr int kNT = 64;                         // output columns per CTA
-constexpr int kStages = 4;
-constexpr int kGemmThreads = 256;               // warp w reads TMEM lanes 32 (w % 4) .., columns 32 (w / 4) ..
+// A plain product of many rows takes all 256 columns in a CTA, which then reads its rows once, in a ring of two stages
+// (two CTAs share an SM with either tile). The line is where four narrow CTAs per 128 rows need a second round, two on
+// each of 152 SMs (a call of K = 256 and of 1024, us, narrow / wide: 9728 rows 29.6 / 31.3 and 53.3 / 55.7, 9729 rows
+// 33.2 / 32.8 and 65.1 / 56.9, 65536 rows 91.9 / 71.7 and 250.6 / 153.2).
+constexpr int kGemmThreads = 256;               // warp w reads TMEM lanes 32 (w % 4) .., column half w / 4
 constexpr int kStageA = kM * kKC * 2;           // 16 KB
-constexpr int kStageB = kNT * kKC * 2;          // 8 KB
-constexpr int kGemmSmem = kStages * (kStageA + kStageB) + 64;  // stages, barriers, TMEM address
+template <int NT>                               // output columns per CTA
+struct GemmTile {
+    static constexpr int kStages = NT == 64 ? 4 : 2;
+    static constexpr int kStageB = NT * kKC * 2;  // 8 KB, 32 KB
+    static constexpr int kSmem = kStages * (kStageA + kStageB) + 64;  // stages, barriers, TMEM address
+};
+constexpr int kNT = 64;                         // of the training products
+constexpr int kWideTiles = 2 * 152 * kNT / kN + 1;  // row tiles
 
 enum Epi : int { EPI_STORE_F32 = 0, EPI_FWD = 1, EPI_BWD = 2 };
 
@@ -191,23 +199,24 @@ __device__ __forceinline__ float dsilu_f(float z) {
     return s * (1.0f + z * (1.0f - s));
 }
 
-template <int EPI>
+template <int EPI, int NT>
 __global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch batch) {
+    constexpr int kStages = GemmTile<NT>::kStages, kStageB = GemmTile<NT>::kStageB;
     extern __shared__ __align__(1024) unsigned char sm[];
-    const GemmArgs& g = batch.g[blockIdx.z / (kN / kNT)];
+    const GemmArgs& g = batch.g[blockIdx.z / (kN / NT)];
     unsigned char* const stA0 = sm;
     unsigned char* const stB0 = sm + kStages * kStageA;
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kStages * (kStageA + kStageB));  // [kStages]
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + kStages);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * kM, n0 = (blockIdx.z % (kN / kNT)) * kNT;
+    const int m0 = blockIdx.x * kM, n0 = (blockIdx.z % (kN / NT)) * NT;
     const int kb = blockIdx.y * g.k_split;
     const int ke = min(g.K, kb + g.k_split);
     const int nc = ke > kb ? (ke - kb) / kKC : 0;
     auto load = [&](int c) {
         const int st = c % kStages;
         load_chunk(stA0 + st * kStageA, g.A, g.lda, m0, kM, g.M, kb + c * kKC);
-        load_chunk(stB0 + st * kStageB, g.B, g.ldb, n0, kNT, kN, kb + c * kKC);
+        load_chunk(stB0 + st * kStageB, g.B, g.ldb, n0, NT, kN, kb + c * kKC);
     };
     for (int c = 0; c < kStages - 1; ++c) {
         if (c < nc) load(c);
@@ -217,7 +226,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch ba
         for (int i = 0; i < kStages; ++i) mbar_init(&bar[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(tslot, kNT);
+    if (warp == 0) tmem_alloc(tslot, NT);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -243,7 +252,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch ba
             const uint32_t a0 = smem_u32(stA0 + (c % kStages) * kStageA), b0 = smem_u32(stB0 + (c % kStages) * kStageB);
 #pragma unroll
             for (int kk = 0; kk < kKC / 16; ++kk)
-                mma_bf16(tmem, smem_desc(a0 + kk * 256, 128, 1024), smem_desc(b0 + kk * 256, 128, 1024), idesc_of(kNT),
+                mma_bf16(tmem, smem_desc(a0 + kk * 256, 128, 1024), smem_desc(b0 + kk * 256, 128, 1024), idesc_of(NT),
                          (c > 0 || kk > 0) ? 1u : 0u);
             mma_commit(&bar[c % kStages]);
         }
@@ -259,10 +268,14 @@ __global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch ba
     ok = __syncthreads_and(ok);
     tc_fence_after();
     if (ok && issued > 0) {
-        const int m = m0 + 32 * (warp & 3) + lane, j0 = n0 + 32 * (warp >> 2);
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * (warp >> 2)), v);
-        if (m < g.M) {
+        const int m = m0 + 32 * (warp & 3) + lane;
+#pragma unroll 1
+        for (int jt = (NT / 2) * (warp >> 2); jt < (NT / 2) * (warp >> 2) + NT / 2; jt += 32) {
+            const int j0 = n0 + jt;
+            float v[32];
+            __syncwarp();
+            tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)jt, v);
+            if (m >= g.M) continue;
             if constexpr (EPI == EPI_STORE_F32) {
                 float4* o = reinterpret_cast<float4*>(g.out_f32 + blockIdx.y * g.part + (long long)m * g.ldo + j0);
 #pragma unroll
@@ -306,27 +319,30 @@ __global__ void __launch_bounds__(kGemmThreads, 2) umma_gemm_kernel(GemmBatch ba
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, kNT);
+        tmem_dealloc(tmem, NT);
     }
 }
 
 // Opt-in shared memory of every GEMM variant on the current device (called before any launch, outside
 // stream capture).
 static cudaError_t set_gemm_attributes() {
-    const void* fns[] = {(const void*)umma_gemm_kernel<EPI_STORE_F32>, (const void*)umma_gemm_kernel<EPI_FWD>,
-                         (const void*)umma_gemm_kernel<EPI_BWD>};
-    for (const void* f : fns) {
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+    const struct { const void* f; int smem; } fns[] = {
+        {(const void*)umma_gemm_kernel<EPI_STORE_F32, kNT>, GemmTile<kNT>::kSmem},
+        {(const void*)umma_gemm_kernel<EPI_STORE_F32, kN>, GemmTile<kN>::kSmem},
+        {(const void*)umma_gemm_kernel<EPI_FWD, kNT>, GemmTile<kNT>::kSmem},
+        {(const void*)umma_gemm_kernel<EPI_BWD, kNT>, GemmTile<kNT>::kSmem}};
+    for (const auto& k : fns) {
+        cudaError_t e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
 // `count` products of one shape in one launch.
-template <int EPI>
+template <int EPI, int NT = kNT>
 static cudaError_t launch_gemm(const GemmBatch& b, int count, int grid_y, cudaStream_t st) {
-    dim3 grid((b.g[0].M + kM - 1) / kM, grid_y, count * (kN / kNT));
-    umma_gemm_kernel<EPI><<<grid, kGemmThreads, kGemmSmem, st>>>(b);
+    dim3 grid((b.g[0].M + kM - 1) / kM, grid_y, count * (kN / NT));
+    umma_gemm_kernel<EPI, NT><<<grid, kGemmThreads, GemmTile<NT>::kSmem, st>>>(b);
     return cudaGetLastError();
 }
 
@@ -1271,7 +1287,9 @@ extern "C" int clr_bf16_gemm_n256(const void* d_a, int64_t lda, const void* d_b,
     GemmArgs& g = b.g[0];
     g.A = static_cast<const bf16*>(d_a); g.lda = lda; g.B = static_cast<const bf16*>(d_b); g.ldb = ldb;
     g.M = (int)M; g.K = (int)K; g.k_split = (int)K; g.out_f32 = d_c; g.ldo = ldc; g.err = err;
-    if (launch_gemm<EPI_STORE_F32>(b, 1, 1, st) != cudaSuccess) return CLR_ERR_CUDA;
+    const bool wide = (M + kM - 1) / kM >= kWideTiles;
+    if ((wide ? launch_gemm<EPI_STORE_F32, kN>(b, 1, 1, st) : launch_gemm<EPI_STORE_F32>(b, 1, 1, st)) != cudaSuccess)
+        return CLR_ERR_CUDA;
     int herr = 0;
     if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return CLR_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return CLR_ERR_CUDA;
