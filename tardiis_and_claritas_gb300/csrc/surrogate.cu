@@ -134,7 +134,6 @@ constexpr int kM = 128, kN = 256, kKC = 64;  // rows per tile, output width, K p
 __host__ __device__ constexpr uint32_t idesc_of(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
 }
-constexpr uint32_t kIdesc = idesc_of(kN);
 
 // The training products are small (2048 x 256 x 256), so a launch's time is a tile's own chain: operands in, MMAs,
 // epilogue. A CTA takes 64 of the 256 output columns (64 CTAs for 2048 rows instead of 16), brings its whole

@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kWaveThreads, 1) wave_cond_warp_kernel(WaveLau
 // The rest of the closure of the photon in `slot` across the warp (closure_rest_warp; called by all 32 lanes):
 // every lane reads the photon and ends with the same state, `owner` writes it back. Returns the photon's next
 // queue, the same in every lane.
-template <class Mode, bool kProv>
+template <class Mode>
 __device__ __forceinline__ int cond_rest_visit(const WaveLaunch& w, const WavePool<Mode>& pool, uint32_t slot, int owner,
                                                unsigned long long* scratch) {
     Ray r = pool.ray[slot];
@@ -600,15 +600,13 @@ __device__ __forceinline__ int cond_rest_visit(const WaveLaunch& w, const WavePo
     const int v = closure_rest_warp(D, r, L.optics(), w.tallies[m.sid].c.cstats, m.pidx, m.cond_kind, &cs, scratch);
     __syncwarp();
     if ((int)(threadIdx.x & 31) == owner) {
-        if constexpr (kProv) {
-            if (w.prov && r.ic == ic0) {  // as the per-lane stage body: survived, or ended by absorption
-                uint4 pv = w.prov[slot];
-                const int type = prov_type(r.wcoh - coh0, r.wmorph - mor0, r.pc.entry_reflections - per0,
-                                           r.pc.internal_reflections - pir0);
-                if (v == 0) prov_event(pv, r.ic, type, m.pidx, vinx, viny, vinz, r.vx, r.vy, r.vz);
-                else if (r.st == 5) prov_mark(pv, r.ic, type, m.pidx);
-                w.prov[slot] = pv;
-            }
+        if (w.prov && r.ic == ic0) {  // as the per-lane stage body: survived, or ended by absorption
+            uint4 pv = w.prov[slot];
+            const int type = prov_type(r.wcoh - coh0, r.wmorph - mor0, r.pc.entry_reflections - per0,
+                                       r.pc.internal_reflections - pir0);
+            if (v == 0) prov_event(pv, r.ic, type, m.pidx, vinx, viny, vinz, r.vx, r.vy, r.vz);
+            else if (r.st == 5) prov_mark(pv, r.ic, type, m.pidx);
+            w.prov[slot] = pv;
         }
         pool.ray[slot] = r;
         pool.lane[slot] = L;
@@ -654,7 +652,7 @@ __global__ void __launch_bounds__(kWaveThreads, 1) wave_cond_diag_kernel(WaveLau
         __syncwarp();
         for (unsigned todo = __ballot_sync(FULL, dest == WQ_COND); todo; todo &= todo - 1u) {
             const int owner = __ffs(todo) - 1;
-            const int next = cond_rest_visit<Mode, true>(w, pool, __shfl_sync(FULL, slot, owner), owner, mine);
+            const int next = cond_rest_visit<Mode>(w, pool, __shfl_sync(FULL, slot, owner), owner, mine);
             if (lane == owner) dest = next;
         }
         wave_push(w, dest, slot);
