@@ -199,15 +199,15 @@ struct SideStream {
 };
 cudaError_t enqueue_particle_precompute(ParticleBuffers& pb, const clr_scene_params& sp, const clr_particle_spec& ps,
                                         const clr_sediment_spec& ss, const SideStream& side, cudaStream_t stream);
-// The meridional advection-diffusion field of sediment model 3 (one cooperative launch, a CTA per bin)
-// into pb.sed_grid and pb.grid_max; pb.merid_* must be allocated (meridional_coef_doubles coefficients).
+// The meridional advection-diffusion field of sediment model 3 (one cooperative launch, a cluster of CTAs per
+// bin) into pb.sed_grid and pb.grid_max; pb.merid_* must be allocated (meridional_coef_doubles coefficients).
 size_t meridional_coef_doubles(int n, int nr, int nz);
 cudaError_t enqueue_meridional_solve(ParticleBuffers& pb, const clr_scene_params& sp, const clr_sediment_spec& ss,
                                      cudaStream_t stream);
 // The part of it after the Mie tables (rates, sediment, node tables); pb's Mie outputs must be ready.
 cudaError_t enqueue_scene_rates(ParticleBuffers& pb, const clr_scene_params& sp, const clr_particle_spec& ps,
                                 const clr_sediment_spec& ss, cudaStream_t stream);
-// The same for n scenarios at once (one launch each for the one-thread rate and majorant kernels);
+// The same for n scenarios at once (one launch each for the rate and majorant kernels);
 // d_scratch: scene_rates_batch_scratch(n) bytes of device memory.
 size_t scene_rates_batch_scratch(int n);
 cudaError_t enqueue_scene_rates_batch(ParticleBuffers* const* pbs, const clr_scene_params* sps,

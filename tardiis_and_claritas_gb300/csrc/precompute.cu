@@ -7,9 +7,10 @@
 // the parallel decomposition changes:
 //  * Mie coefficients: one block per size bin, the three recurrences in a warp each
 //    in shared memory instead of a global scratch array;
-//  * phase pdf: one thread per (angle, group of 4 bins) sharing the angular
-//    pi_n/tau_n recurrence across the group (the recurrence depends only on the
-//    angle), instead of one thread per (bin, angle) recomputing it;
+//  * phase pdf: the angular functions pi_n/tau_n, which depend only on the angle and
+//    the order, come from a table made once, instead of a recurrence in every
+//    (bin, angle) thread; where that table would be too large, threads run it, for
+//    four bins at a time where there are many;
 //  * Schiller-Naumann radial slip: one thread per (bin, radius) instead of one
 //    thread for everything; the serial prefix sums and quadrature stay serial
 //    per bin so their rounding is unchanged.
@@ -1037,8 +1038,8 @@ __global__ void sediment_node_kernel(const double* __restrict__ grid, const doub
 // volumes with no-flux walls, red-black SOR, per-bin mass renormalisation every 20 iterations and at every
 // convergence check, stopping at the first check (after at least min(1000, max) iterations) where the
 // largest relative residual over all bins is within tolerance (CLARITAS/CLARITAS.py:4040-4215, driven by
-// :6451-6725, one launch per half-sweep). Here one cooperative launch does all of it: a CTA per bin keeps
-// its bin's plane in shared memory; the bins meet only at the checks (a bounded grid barrier) to agree on
+// :6451-6725, one launch per half-sweep). Here one cooperative launch does all of it: a cluster of CTAs
+// per bin keeps its bin's plane in shared memory; the bins meet only at the checks (a bounded grid barrier) to agree on
 // the largest residual. Every cell value, sum order and stopping iteration is the reference's.
 
 // free-surface height and slope at radius r (:4046-4057)
@@ -1682,8 +1683,8 @@ cudaError_t enqueue_scene_rates(ParticleBuffers& pb, const clr_scene_params& sp,
 
 size_t scene_rates_batch_scratch(int n) { return (size_t)n * (sizeof(TransportJob) + sizeof(MajorantJob)) + 256; }
 
-// The same for n scenarios: the one-thread rate and majorant kernels of all scenarios run as one launch
-// each (a thread per scenario); the sediment bins and node tables stay per scenario. `d_scratch` holds
+// The same for n scenarios: the rate and majorant kernels of all scenarios run as one launch each (a warp
+// per scenario); the sediment bins and node tables stay per scenario. `d_scratch` holds
 // scene_rates_batch_scratch(n) bytes of device memory for the job descriptions.
 cudaError_t enqueue_scene_rates_batch(ParticleBuffers* const* pbs, const clr_scene_params* sps,
                                       const clr_particle_spec* pss, const clr_sediment_spec* sss, int n,

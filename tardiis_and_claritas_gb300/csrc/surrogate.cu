@@ -2,14 +2,16 @@
 // counterpart: the reference answers every scenario query with a full Monte Carlo run).
 //
 // Network: 6 -> 256 -> 256 -> 256 -> 256 -> 3, SiLU after each hidden layer, BF16 weights and
-// activations, FP32 accumulation, FP32 master weights with Adam. The three 256x256 layers run on the
-// 5th-generation tensor cores: one GEMM kernel computes C[M][256] = A[M][K] . B[256][K]^T with both
+// activations, FP32 accumulation, FP32 master weights with Adam. In training the three 256x256 layers run
+// on the 5th-generation tensor cores: one GEMM kernel computes C[M][256] = A[M][K] . B[256][K]^T with both
 // operands K-major BF16, staged through shared memory in the canonical no-swizzle core-matrix layout
-// and multiplied by tcgen05.mma (M=128, N=256, K=16 per instruction) into a TMEM accumulator, which
-// the epilogue reads back with tcgen05.ld. The same kernel serves the forward layers (bias + SiLU
-// epilogue), the backward-data products (SiLU-derivative epilogue) and the weight gradients (split-K
-// over the batch, FP32 atomics). The thin first (6 -> 256) and last (256 -> 3) layers, the loss, the
-// bias gradients and the Adam update are CUDA-core kernels.
+// and multiplied by tcgen05.mma (M=128, N=64, K=16 per instruction; a CTA makes 128 rows of 64 columns)
+// into a TMEM accumulator, which the epilogue reads back with tcgen05.ld. The same kernel serves the
+// forward layers (bias + SiLU epilogue), the backward-data products (SiLU-derivative epilogue) and the
+// weight gradients (split-K over the batch into partial sums, which Adam adds in a fixed order). The thin
+// first (6 -> 256) and last (256 -> 3) layers, the loss (added by atomics, so that its last bits depend on
+// the order of the blocks), the bias gradients and the Adam update are CUDA-core kernels. Inference is one
+// kernel of its own (mlp_infer_kernel) with every product on the tensor cores.
 #include <cstdint>
 #include <cstring>
 #include <cmath>
@@ -608,8 +610,8 @@ __global__ void pack_kernel(const float* __restrict__ params, PackArgs pa) {
     if (p < (int)kParams) pack_one(pa, p, params[p]);
 }
 
-// Adam (bias-corrected) on every parameter, then the gradient is cleared and the BF16 copies refreshed. hp: per
-// step of the call the learning rate and the two bias corrections.
+// Adam (bias-corrected) on every parameter, whose gradient it adds up from the step's partial sums; then the BF16
+// copies are refreshed. hp: per step of the call the learning rate and the two bias corrections.
 __global__ void adam_kernel(float* params, GradParts G, float* m1, float* m2, const StepArgs* __restrict__ step,
                             const float4* __restrict__ hp, PackArgs pa) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -636,7 +638,7 @@ __global__ void adam_kernel(float* params, GradParts G, float* m1, float* m2, co
 // 128 columns, the accumulator the other 256), from where tcgen05.mma takes its A operand, which leaves shared
 // memory to the weights: a ring of three half layers (64 KB each, one bulk copy), refilled as each half's MMAs end.
 // With the activations in shared memory, one weight buffer and each layer's MMAs, copy and epilogue one after the
-// other, 65536 queries took 52 us; now 40.4 us (a call 79.6 -> 71.3 us). What is left is the chain half of MMAs ->
+// other, 65536 queries took 52 us; now 40.4 us (a call 80.8 -> 74.1 us). What is left is the chain half of MMAs ->
 // half epilogue of a tile, about 10 us, of which 131072 tanh on the multi-function unit take 4.3.
 constexpr int kInferWarps = 16;                  // epilogue warps: TMEM lane quarter w % 4, 32 columns of each half
 constexpr int kInferThreads = 32 * (kInferWarps + 1);  // and one warp that issues copies and MMAs
