@@ -9,7 +9,7 @@ merit 1 / (relative SE^2 x time), so the speed ratio at equal tally error is
 measured, not assumed.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--workload full|small|sweep]
-  python bench.py --impl reference ...   # the reference's own CPU implementation
+  python bench.py --impl reference ...   # the reference's own CPU implementation, where its source is at hand
 
 With --workload sweep a step builds and traces the 512-scenario batched sweep (per-scenario Mie
 tables, rates and photon counts log-uniform over 1e5-1e7) and the metric is scenarios/s.
@@ -556,6 +556,12 @@ class CpuReference:
 def run_reference_arm(args, rank: int, world: int):
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    import oracle_harness as H
+    if not H.reference_available():  # the restatement is this repository's code: its time is not the reference's
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's source is not in this tree, and neither is a host build of it"}), flush=True)
+        return
     threads = os.cpu_count() or 1
     name = args.workload
     if name == "surrogate":
@@ -610,8 +616,7 @@ def run_reference_arm(args, rank: int, world: int):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32/f64",
             "data": "synthetic (seeded)", "config": cfg_line,
             "cpu_baseline": {"value": value, "unit": "photons/s", "cores": threads, "kind": ref.kind,
-                             "build": "the reference's CUDA_SRC as host C++, -O3, OpenMP over photons"
-                             if ref.kind == "reference" else "the CPU restatement, -O2, OpenMP over photons",
+                             "build": "the reference's CUDA_SRC as host C++, -O3, OpenMP over photons",
                              "sample": f"{n} photons of the same workload per step, {args.steps} steps"},
             "tally_error": channel_error(tallies, total_t),
             "e2e": {"value": value, "unit": "photons/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
